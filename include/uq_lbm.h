@@ -244,8 +244,11 @@ LBM_API lbm_status lbm_batch_profile(lbm_batch *b, int n_steps, double *phase_ms
  * ms_per_step (one per candidate) may be NULL. */
 LBM_API lbm_status lbm_batch_autotune(lbm_batch *b, const int *candidates, int n_candidates, int steps, int *chosen,
                                       double *ms_per_step);
-/* Kernel launches one step of the batch issues. */
+/* Kernel launches of one step taken phase by phase, every part apart: what
+ * lbm_batch_profile times and a batch without use_graph runs ... */
 LBM_API int lbm_batch_launches_per_step(lbm_batch *b, int want_residual);
+/* ... and of one step replayed from a graph, which merges the parts. */
+LBM_API int lbm_batch_graph_launches(lbm_batch *b, int want_residual);
 /* Lattice updates (nodes) one step of the whole batch performs. */
 LBM_API long long lbm_batch_nodes(lbm_batch *b);
 LBM_API void *lbm_batch_stream(lbm_batch *b);

@@ -86,15 +86,19 @@ struct PreparedSample {
 
 HostSample derive(const lbm_config &c, const lbm_init &in);
 void prepare_sample(const HostSample &h, int prec, PreparedSample &out);
-// append the tx x ty tiles of one sample (flags in pitch layout, sample
-// flags sflags for its periodic axes) with the given sample index; gid
+// append the tx x ty tiles of one sample (p: its parameters; flags in pitch
+// layout) with the given sample index, each with its kind (see Tile); gid
 // numbers continue from out.size()
-void cut_tiles(const uint8_t *flags, int pitch, int nx, int ny, int tx, int ty, int sflags, int gx, int sample,
-               std::vector<Tile> &out);
+void cut_tiles(const uint8_t *flags, const SampleParams &p, int tx, int ty, int sample, std::vector<Tile> &out);
+// the wall nodes whose factor a general tile of the sample reads (sweep tiles
+// form the factors of straight walls themselves); tiles: the sample's, as
+// cut_tiles made them
+void needed_walls(const SampleParams &p, int tx, int ty, const Tile *tiles, const std::vector<WallNode> &walls,
+                  std::vector<WallNode> &out);
 // TMA descriptors of one sample (MAPS_PER_SAMPLE of them): stage buffers 2
-// and 3 with the stencil halo box, and the state with the tile's own box
-void encode_stage_maps(int prec, const SampleParams &p, unsigned char *state, unsigned char *buf2,
-                       unsigned char *buf3, int tx, int ty, CUtensorMap *maps);
+// and 3, each with the stencil kernels' three box shapes
+void encode_stage_maps(int prec, const SampleParams &p, unsigned char *buf2, unsigned char *buf3, int tx, int ty,
+                       CUtensorMap *maps);
 void check_tile_shape(int x, int y);
 int round_up(int v, int m);
 
@@ -106,84 +110,121 @@ struct TileRun {
 
 // Device pointers and lengths of the packed lists one step launches over.
 // The pointwise phase runs over the tiles of each RKMETHOD in sample order;
-// the stencil phases over the same tiles as three runs, the simple tiles,
-// the wrap tiles and the rest, one kernel per run, each compiled for its
-// kind of tile alone.
+// the stencil phases over the same tiles as two runs, the sweep tiles and
+// the general tiles, one kernel per run.
 struct StepLists {
-    TileRun pointwise[4];                           // tiles by RKMETHOD, sample order
-    TileRun simple[4], wrap[4], general[4];         // the same tiles by kind
-    TileRun rk3_simple, rk3_wrap, rk3_general;      // RK3 tiles (final stencil phase)
+    TileRun pointwise[4];            // tiles by RKMETHOD, sample order
+    TileRun sweep[4], general[4];    // the same tiles by kind
+    TileRun rk3_sweep, rk3_general;  // RK3 tiles (final stencil phase)
+    // the wall nodes that general tiles read (WallNode lists)
     const WallNode *walls_all = nullptr, *walls_rk3 = nullptr;
     int n_walls_all = 0, n_walls_rk3 = 0;
-    // the samples, for copying buffer 2's ghost columns (SampleParams::gx)
-    // after the pointwise phase
+    // for a step taken phase by phase: the sweep runs' kinds (tile_rank: 0,
+    // 1, the rest 2), every wall node, and the samples
+    int kinds[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}}, rk3_kinds[2] = {0, 0};
+    const WallNode *every_wall = nullptr, *every_wall_rk3 = nullptr;
+    int n_every_wall = 0, n_every_wall_rk3 = 0;
     const SampleParams *samples = nullptr;
     int nsamples = 0;
     bool any_ghost = false;
 };
 
-// A device list of n tiles whose first ns are simple and next nw wrap
-// tiles, as three runs.
-inline void split_runs(const Tile *p, int n, int ns, int nw, TileRun &simple, TileRun &wrap, TileRun &general)
+// A device list of n tiles whose first ns are sweep tiles, as two runs.
+inline void split_runs(const Tile *p, int n, int ns, TileRun &sweep, TileRun &general)
 {
-    simple.p = p;
-    simple.n = ns;
-    wrap.p = p ? p + ns : nullptr;
-    wrap.n = nw;
-    general.p = p ? p + ns + nw : nullptr;
-    general.n = n - ns - nw;
+    sweep.p = p;
+    sweep.n = ns;
+    general.p = p ? p + ns : nullptr;
+    general.n = n - ns;
 }
 
-// Reorder a host tile list by kind, simple tiles first, then wrap tiles,
-// then the rest (each kind keeps its order); ns, nw: how many are simple
-// and wrap tiles.
-inline void order_by_kind(std::vector<Tile> &v, int &ns, int &nw)
+// Reorder a host tile list by kind (tile_rank; each kind keeps its order);
+// ns: how many are sweep tiles, kinds: how many of the first two kinds.
+inline void order_by_kind(std::vector<Tile> &v, int &ns, int *kinds = nullptr)
 {
-    auto mid = std::stable_partition(v.begin(), v.end(), [](const Tile &t) { return tile_simple(t); });
-    auto end = std::stable_partition(mid, v.end(), [](const Tile &t) { return tile_wrap(t); });
-    ns = (int)(mid - v.begin());
-    nw = (int)(end - mid);
+    std::stable_sort(v.begin(), v.end(), [](const Tile &a, const Tile &b) { return tile_rank(a) < tile_rank(b); });
+    int n[4] = {0, 0, 0, 0};
+    for (const Tile &t : v) ++n[tile_rank(t)];
+    ns = n[0] + n[1] + n[2];
+    if (kinds) {
+        kinds[0] = n[0];
+        kinds[1] = n[1];
+    }
 }
 
 template <class S, class C>
-void stencil_runs(const KArgs<S> &a, int phase, int m, const TileRun &s, const TileRun &w, const TileRun &g,
-                  cudaStream_t st)
+void stencil_runs(const KArgs<S> &a, int phase, int m, const TileRun &s, const TileRun &g, cudaStream_t st)
 {
-    if (s.n) CU((launch_phase<S, C>(a, phase, m, s.p, s.n, nullptr, 0, st, FLUX_SIMPLE)));
-    if (w.n) CU((launch_phase<S, C>(a, phase, m, w.p, w.n, nullptr, 0, st, FLUX_WRAP)));
+    if (s.n) CU((launch_phase<S, C>(a, phase, m, s.p, s.n, nullptr, 0, st, FLUX_SWEEP)));
     if (g.n) CU((launch_phase<S, C>(a, phase, m, g.p, g.n, nullptr, 0, st, FLUX_GENERAL)));
 }
 
-// One step: pointwise stages, walls, first stencil phase, and for RK3 the
-// walls of buffer 3 and the final stencil phase.  ev (optional) receives
-// events [0] start, after pointwise, walls 2, phase 1, walls 3, phase 2.
+// One step: pointwise stages, first stencil phase, and for RK3 the final
+// stencil phase; wall factors before a stencil phase with general tiles that
+// read some.
 template <class S, class C>
-void enqueue_step_phases(const KArgs<S> &a, const StepLists &l, cudaStream_t st, cudaEvent_t *ev = nullptr)
+void enqueue_step(const KArgs<S> &a, const StepLists &l, cudaStream_t st)
 {
+    for (int m = 0; m < 4; ++m)
+        if (l.pointwise[m].n) CU((launch_phase<S, C>(a, 0, m, l.pointwise[m].p, l.pointwise[m].n, nullptr, 0, st)));
+    CU((launch_phase<S, C>(a, 3, 0, nullptr, 0, l.walls_all, l.n_walls_all, st)));
+    for (int m = 0; m < 4; ++m) stencil_runs<S, C>(a, 1, m, l.sweep[m], l.general[m], st);
+    if (l.rk3_sweep.n || l.rk3_general.n) {
+        CU((launch_phase<S, C>(a, 4, 1, nullptr, 0, l.walls_rk3, l.n_walls_rk3, st)));
+        stencil_runs<S, C>(a, 2, 1, l.rk3_sweep, l.rk3_general, st);
+    }
+}
+
+// kernels that enqueue_step launches
+inline int step_launches(const StepLists &l)
+{
+    int n = l.n_walls_all ? 1 : 0;
+    for (int m = 0; m < 4; ++m) n += (l.pointwise[m].n ? 1 : 0) + (l.sweep[m].n ? 1 : 0) + (l.general[m].n ? 1 : 0);
+    if (l.rk3_sweep.n || l.rk3_general.n)
+        n += (l.n_walls_rk3 ? 1 : 0) + (l.rk3_sweep.n ? 1 : 0) + (l.rk3_general.n ? 1 : 0);
+    return n;
+}
+
+// The same step phase by phase, every part in launches of its own (the ghost
+// columns, the wall factors, each kind of tile): what lbm_batch_profile times
+// and a batch without a graph runs.  Same results, bit for bit.  ev
+// (optional) receives events [0] start, after pointwise, walls 2, phase 1,
+// walls 3, phase 2.
+template <class S, class C>
+void enqueue_step_phased(KArgs<S> a, const StepLists &l, cudaStream_t st, cudaEvent_t *ev = nullptr)
+{
+    a.phased = 1;
+    auto kinds = [&](int phase, int m, const TileRun &s, const int *k, const TileRun &g) {
+        const TileRun run[3] = {{s.p, k[0]}, {s.p + k[0], k[1]}, {s.p + k[0] + k[1], s.n - k[0] - k[1]}};
+        for (const TileRun &r : run) stencil_runs<S, C>(a, phase, m, r, TileRun{}, st);
+        stencil_runs<S, C>(a, phase, m, TileRun{}, g, st);
+    };
     if (ev) CU(cudaEventRecord(ev[0], st));
     for (int m = 0; m < 4; ++m)
         if (l.pointwise[m].n) CU((launch_phase<S, C>(a, 0, m, l.pointwise[m].p, l.pointwise[m].n, nullptr, 0, st)));
     if (l.any_ghost) CU(launch_fill_ghosts<S>(l.samples, 0, l.nsamples, a.buf2, nullptr, st));
     if (ev) CU(cudaEventRecord(ev[1], st));
-    CU((launch_phase<S, C>(a, 3, 0, nullptr, 0, l.walls_all, l.n_walls_all, st)));
+    CU((launch_phase<S, C>(a, 3, 0, nullptr, 0, l.every_wall, l.n_every_wall, st)));
     if (ev) CU(cudaEventRecord(ev[2], st));
-    for (int m = 0; m < 4; ++m) stencil_runs<S, C>(a, 1, m, l.simple[m], l.wrap[m], l.general[m], st);
-    const bool rk3 = l.rk3_simple.n || l.rk3_wrap.n || l.rk3_general.n;
+    for (int m = 0; m < 4; ++m) kinds(1, m, l.sweep[m], l.kinds[m], l.general[m]);
     if (ev) CU(cudaEventRecord(ev[3], st));
-    if (rk3) CU((launch_phase<S, C>(a, 4, 1, nullptr, 0, l.walls_rk3, l.n_walls_rk3, st)));
+    const bool rk3 = l.rk3_sweep.n || l.rk3_general.n;
+    if (rk3) CU((launch_phase<S, C>(a, 4, 1, nullptr, 0, l.every_wall_rk3, l.n_every_wall_rk3, st)));
     if (ev) CU(cudaEventRecord(ev[4], st));
-    if (rk3) stencil_runs<S, C>(a, 2, 1, l.rk3_simple, l.rk3_wrap, l.rk3_general, st);
+    if (rk3) kinds(2, 1, l.rk3_sweep, l.rk3_kinds, l.rk3_general);
     if (ev) CU(cudaEventRecord(ev[5], st));
 }
 
-inline int step_launches(const StepLists &l)
+// kernels that enqueue_step_phased launches
+inline int phased_launches(const StepLists &l)
 {
-    int n = l.any_ghost ? 1 : 0;
-    for (int m = 0; m < 4; ++m)
-        n += (l.pointwise[m].n ? 1 : 0) + (l.simple[m].n ? 1 : 0) + (l.wrap[m].n ? 1 : 0) + (l.general[m].n ? 1 : 0);
-    n += l.n_walls_all ? 1 : 0;
-    if (l.rk3_simple.n || l.rk3_wrap.n || l.rk3_general.n)
-        n += (l.n_walls_rk3 ? 1 : 0) + (l.rk3_simple.n ? 1 : 0) + (l.rk3_wrap.n ? 1 : 0) + (l.rk3_general.n ? 1 : 0);
+    auto kinds = [](const TileRun &s, const int *k, const TileRun &g) {
+        return (k[0] ? 1 : 0) + (k[1] ? 1 : 0) + (s.n > k[0] + k[1] ? 1 : 0) + (g.n ? 1 : 0);
+    };
+    int n = (l.any_ghost ? 1 : 0) + (l.n_every_wall ? 1 : 0);
+    for (int m = 0; m < 4; ++m) n += (l.pointwise[m].n ? 1 : 0) + kinds(l.sweep[m], l.kinds[m], l.general[m]);
+    if (l.rk3_sweep.n || l.rk3_general.n)
+        n += (l.n_every_wall_rk3 ? 1 : 0) + kinds(l.rk3_sweep, l.rk3_kinds, l.rk3_general);
     return n;
 }
 

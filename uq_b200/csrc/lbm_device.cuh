@@ -2,10 +2,12 @@
 //
 // Every function restates a piece of the reference FP64 CPU solver
 // CODE/C++/VS2010/simLB/simLB/cpuLBM.cpp (cited per function) for the GPU's
-// structure-of-arrays layout: per sample, 26 planes (f_0..f_12, h_0..h_12),
-// each plane ny rows of `pitch` elements, x fastest.  Templates take the
-// storage type S (double or float) and the compute type C; moment sums are
-// always accumulated in double.
+// layout: per sample, 13 planes, one per direction, each ny rows of `pitch`
+// nodes, x fastest; a node of plane i is the pair (f_i, h_i), so that f and h,
+// which every stage treats alike, move in one 8- (FP32) or 16-byte (FP64)
+// access and are the two lanes of the packed FP32 arithmetic.  Templates take
+// the storage type S (double or float) and the compute type C; moment sums
+// are always accumulated in double.
 #pragma once
 
 #include <cstdint>
@@ -13,7 +15,14 @@
 namespace uqlbm {
 
 constexpr int NQ = 13;
-constexpr int NPL = 26;  // f and h planes
+constexpr int NPL = 26;  // f and h values of a node
+
+// element of direction i (f: fh = 0, h: fh = 1) at node offset o (in the
+// plane), relative to the sample's plane 0
+__host__ __device__ constexpr long long el(int i, int fh, long long plane, long long o)
+{
+    return 2 * (i * plane + o) + fh;
+}
 
 // node-flag byte: cell type in bits 0-1 (0 fluid, 1 permanent, 2 solid);
 // bits 2-5 say whether the 5-point x / y stencil of the node meets a solid
@@ -34,8 +43,8 @@ struct SampleParams {
     int rk, fm;          // RKMETHOD, FMETHOD
     int ntile;           // tiles of this sample in the full tile list
     int first_tile;
-    long long state_off; // element offset of plane 0 in every state buffer
-    long long plane;     // elements per plane
+    long long state_off; // element offset of plane 0 in every state buffer (even)
+    long long plane;     // nodes per plane
     long long node_off;  // offset into per-node arrays
     int xoff, yoff;      // offsets into the per-column / per-row spacing tables
     double R, bR, K, Tc, inv_sRTc, RTc, mu, Pr, dt, c;
@@ -44,13 +53,14 @@ struct SampleParams {
     // (rho0, 0, 0, T0); rho0 = shref = 0 (full storage) on the FP64 path.
     double rho0, T0n, shref;  // T0n = T0 / Tc
     double inv_mu, two_over_bR;
-    int wide;  // FP32 WENO5 weights in the range-safe form (see weno5)
+    int wide;  // FP32 WENO5 weights in the range-safe form (see weno_face)
+    double eps1;  // FP64: WENO5's epsilon for values not scaled by |e|, 1e-6 / c^2
     // ghost columns of the stage buffers (0 or GHOST_X): x-periodic samples
     // keep, left and right of every row of buffers 2 and 3, the periodic
     // images of the gx columns at the other edge, so the staged halo boxes
     // of tiles at those edges load them as they load any interior node.
     // Rows stay aligned (pitch >= nx + 2 gx, a multiple of 32): the right
-    // ghosts follow the row, the left ones are the last gx elements of the
+    // ghosts follow the row, the left ones are the last gx nodes of the
     // row before (the sample's region starts GHOST_SLACK elements before
     // plane 0 for the first row's).  The per-node arrays have no ghosts.
     int gx;
@@ -66,21 +76,30 @@ constexpr int GHOST_SLACK = 32;  // state elements before plane 0 of a sample wi
 struct Tile {
     int sample;
     int x0, y0;
-    int gid;  // index of the tile in the batch's full tile list; bit 30: simple
+    int gid;   // index of the tile in the batch's full tile list
+    int kind;  // TILE_* bits
+    int pad[3];
 };
 
-// A simple tile lies at least 3 nodes inside its domain and neither it nor
-// its 3-node halo holds a solid/permanent node or a node whose stencil meets
-// a solid or an edge: every flux it needs comes straight from the staged box.
-// A wrap tile is a full tile that would be simple but for a periodic edge:
-// its halo crosses it (along a periodic axis) and holds only plain fluid
-// nodes, so once the periodic images are copied into the staged box every
-// flux comes from the box as in a simple tile.
-constexpr int TILE_SIMPLE = 1 << 30;
-constexpr int TILE_WRAP = 1 << 29;
-__host__ __device__ inline int tile_gid(const Tile &t) { return t.gid & (TILE_WRAP - 1); }
-__host__ __device__ inline bool tile_simple(const Tile &t) { return (t.gid & TILE_SIMPLE) != 0; }
-__host__ __device__ inline bool tile_wrap(const Tile &t) { return (t.gid & TILE_WRAP) != 0; }
+// Kinds of tiles in the stencil phases.  A sweep tile's fluxes all come from
+// its staged box, line by line (see k_flux): every node of the tile and its
+// 3-node halo is plain fluid, or the exceptions are of the forms that are
+// filled into the box first (TILE_FIX): a clamped or periodic domain edge,
+// permanent nodes, a straight wall (row 0 or row ny - 1 solid in all the
+// columns the tile sees; TILE_WALLS, TILE_WALLN).  The other tiles (solids
+// elsewhere, mirror edges) are general: node flags choose per flux.
+constexpr int TILE_SWEEP = 1, TILE_FIX = 2, TILE_WALLS = 4, TILE_WALLN = 8;
+constexpr int TILE_FM_SHIFT = 4;  // 2 bits: 0 NND, 1 WENO5, 2 WENO5 with the range-safe weights
+constexpr int TILE_GHOST = 64;    // the sample has ghost columns
+constexpr int TILE_WRAP = 128;    // a TILE_FIX tile that only wraps (no clamped edge, fixed node or wall)
+__host__ __device__ inline bool tile_sweep(const Tile &t) { return (t.kind & TILE_SWEEP) != 0; }
+// order of the tiles in a stencil run: tiles to complete (the longer ones)
+// first, then those that only wrap, then plain ones; general tiles last
+__host__ __device__ inline int tile_rank(const Tile &t)
+{
+    return !(t.kind & TILE_SWEEP) ? 3 : (t.kind & TILE_WRAP) ? 1 : (t.kind & TILE_FIX) ? 0 : 2;
+}
+__host__ __device__ inline int tile_fm(int kind) { return (kind >> TILE_FM_SHIFT) & 3; }
 
 // lattice (setupVars, cpuLBM.cpp:376-388) in units of c, its signs, and the
 // reflection maps of mirIndex (cpuLBM.cpp:1147-1169)
@@ -144,18 +163,34 @@ __device__ __forceinline__ float2 xfma(float2 a, float2 b, float2 c) { return __
 __device__ __forceinline__ float2 xneg(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 xmin(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
 
+// and on a pair of FP64 values, lane by lane
+__device__ __forceinline__ double2 xmul(double2 a, double2 b) { return make_double2(xmul(a.x, b.x), xmul(a.y, b.y)); }
+__device__ __forceinline__ double2 xadd(double2 a, double2 b) { return make_double2(xadd(a.x, b.x), xadd(a.y, b.y)); }
+__device__ __forceinline__ double2 xsub(double2 a, double2 b) { return make_double2(xsub(a.x, b.x), xsub(a.y, b.y)); }
+__device__ __forceinline__ double2 xfma(double2 a, double2 b, double2 c)
+{
+    return make_double2(xfma(a.x, b.x, c.x), xfma(a.y, b.y, c.y));
+}
+
+// the (f, h) pair of a storage or compute type
+template <class C>
+struct PairOf;
+template <>
+struct PairOf<float> { using type = float2; };
+template <>
+struct PairOf<double> { using type = double2; };
+template <class C>
+using Pair = typename PairOf<C>::type;
+__device__ __forceinline__ float2 make_pair2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 make_pair2(double a, double b) { return make_double2(a, b); }
+
 // a constant in the arithmetic type (both lanes of a pair)
 template <class C>
 __device__ __forceinline__ C kc(double v) { return C(v); }
 template <>
 __device__ __forceinline__ float2 kc<float2>(double v) { return make_float2((float)v, (float)v); }
-// FP32 arithmetic, scalar or packed
-template <class C>
-struct IsF32 { static constexpr bool value = false; };
 template <>
-struct IsF32<float> { static constexpr bool value = true; };
-template <>
-struct IsF32<float2> { static constexpr bool value = true; };
+__device__ __forceinline__ double2 kc<double2>(double v) { return make_double2(v, v); }
 
 // ------------------------------------------------------------ equilibria
 // equilibrium2D (cpuLBM.cpp:785-844) with the polynomials of
@@ -594,16 +629,18 @@ __device__ __forceinline__ Macro macro_from_sums(double r, double rux, double ru
 {
     // stored deviations: add the rest state's rho0 and sum of h (0 when the
     // state is stored in full)
-    r = sp.rho0 + r;
-    sh = sp.shref + sh;
+    // every operation explicitly rounded: each kernel gives a node the same
+    // moments
+    r = __dadd_rn(sp.rho0, r);
+    sh = __dadd_rn(sp.shref, sh);
     Macro m;
-    const double ir = 1.0 / r;
+    const double ir = __drcp_rn(r);
     m.rho = r;
-    m.ux = rux * ir;
-    m.uy = ruy * ir;
-    const double usq = m.ux * m.ux + m.uy * m.uy;
-    m.T = (sh * ir - 0.5 * usq) * sp.two_over_bR;
-    m.p = r * sp.R * m.T;
+    m.ux = __dmul_rn(rux, ir);
+    m.uy = __dmul_rn(ruy, ir);
+    const double usq = __fma_rn(m.uy, m.uy, __dmul_rn(m.ux, m.ux));
+    m.T = __dmul_rn(__fma_rn(sh, ir, __dmul_rn(-0.5, usq)), sp.two_over_bR);
+    m.p = __dmul_rn(__dmul_rn(r, sp.R), m.T);
     if (sp.visc == 0) {
         m.q = m.p * sp.inv_mu;  // 1/tau_f = p/mu
     } else {
@@ -635,6 +672,43 @@ __device__ __forceinline__ int bc_index(const SampleParams &sp, int i, int pm, i
 }
 
 // -------------------------------------------------------------- NND, WENO5
+// Reconstructions of one face, f and h together as the lanes of a pair, from
+// upwind-ordered values s0..s4 (NND: the middle three).  Everything that
+// depends on one or three neighbouring values only is a function of its own,
+// so that the faces of a line form it once (line_diffs); a single face
+// (face5) takes the same operations, so the same bits.
+//
+// FP32 works on the values times |e|, as the reference does.  These flows
+// amplify rounding by orders of magnitude over tens of steps, so the
+// operations and their order are fixed: results do not change with the
+// kernel's structure.  FP64 has room for a cheaper form on the differences
+// of the unscaled values (below).
+
+// what a direction's component along the axis gives a face: |e| (FP32), or
+// epsilon / |e|^2 (FP64, whose flux differences are multiplied by |e| later)
+template <class C>
+struct FaceArg;
+template <>
+struct FaceArg<float> {
+    float2 ae, aeh;  // |e|, |e| / 2
+};
+template <>
+struct FaceArg<double> {
+    double2 eps;
+};
+template <class C>
+__device__ __forceinline__ FaceArg<C> face_arg(const SampleParams &sp, int comp)
+{
+    const bool two = comp == 2 || comp == -2;
+    if constexpr (sizeof(C) == 4) {
+        const float c = (float)sp.c, ae = two ? 2.f * c : c;
+        return FaceArg<C>{make_float2(ae, ae), make_float2(0.5f * ae, 0.5f * ae)};
+    } else {
+        const double e = two ? 0.25 * sp.eps1 : sp.eps1;
+        return FaceArg<C>{make_double2(e, e)};
+    }
+}
+
 // minmod with the reference's case order (cpuLBM.cpp:1130-1145): same
 // signs -> the smaller magnitude (equal magnitudes mean a == b), else 0
 template <class C>
@@ -642,102 +716,251 @@ __device__ __forceinline__ C minmod(C a, C b)
 {
     return a * b > C(0) ? (fabs(a) < fabs(b) ? a : b) : C(0);
 }
-// lane-wise on the packed pair (f, h) of one face
-template <>
-__device__ __forceinline__ float2 minmod<float2>(float2 a, float2 b)
-{
-    return make_float2(minmod<float>(a.x, b.x), minmod<float>(a.y, b.y));
-}
 
-// NND (cpuLBM.cpp:1328-1356) on the 3 upwind-ordered values s0, s1, s2
-template <class C>
-__device__ __forceinline__ C nnd3(C ae, C s0, C s1, C s2)
-{
-    const C c = xmul(ae, s1);
-    return xfma(kc<C>(0.5), minmod<C>(xfma(ae, s2, xneg(c)), xfma(xneg(ae), s0, c)), c);
-}
-
-// one division per face (the FP64 path keeps it correctly rounded)
-__device__ __forceinline__ double face_div(double n, double d) { return n / d; }
-// FP32: n times the approximate reciprocal of d (PTX rcp.approx, then one
-// correctly rounded product).  Inline PTX, so that no compiled instance may
-// lower the division another way: a face then rounds the same in every
-// kernel that reconstructs it.  d here is a positive normal number (a sum
-// of weights, or eps + b_k).
+// FP32 reciprocal: PTX rcp.approx, inline, so that no compiled instance may
+// lower a division another way: a face then rounds the same in every kernel
+// that reconstructs it.  d is a positive normal number (a sum of weights, or
+// eps + b_k).
 __device__ __forceinline__ float rcp_approx(float d)
 {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return r;
 }
-__device__ __forceinline__ float face_div(float n, float d) { return __fmul_rn(n, rcp_approx(d)); }
+// the quotients of both lanes: FP32 by two reciprocals; FP64 by one division
+// of the product of the denominators (a division costs as much as ten
+// products; the products of two denominators stay far inside the FP64 range)
 __device__ __forceinline__ float2 face_div(float2 n, float2 d)
 {
     return __fmul2_rn(n, make_float2(rcp_approx(d.x), rcp_approx(d.y)));
 }
+__device__ __forceinline__ double2 face_div(double2 n, double2 d)
+{
+    const double r = __drcp_rn(xmul(d.x, d.y));
+    return make_double2(xmul(xmul(n.x, d.y), r), xmul(xmul(n.y, d.x), r));
+}
 
 // WENO5 (cpuLBM.cpp:1358-1403): Jiang-Shu indicators b_k, linear weights
-// 1/10, 6/10, 3/10, epsilon 1e-6, on |e| times the upwind-ordered values.
-// The nonlinear weights d_k/(eps+b_k)^2 normalised by their sum are formed
-// as d_k prod_{j!=k} (eps+b_j)^2 over the same sum (one division per face).
-// That fourth power (times the candidate values in the numerator) leaves
-// the FP32 range on dimensional data; for samples whose scales allow that
+// 1/10, 6/10, 3/10, epsilon 1e-6.  The nonlinear weights d_k/(eps+b_k)^2
+// normalised by their sum are formed as d_k prod_{j!=k} (eps+b_j)^2 over the
+// same sum (one division per face).  That fourth power leaves the FP32 range
+// on dimensional data; for samples whose scales allow that
 // (SampleParams::wide, set on the host) the FP32 weights are formed as
 // d_k (m/(eps+b_k))^2 instead, m the smallest eps+b_j, each ratio in (0, 1].
-template <class C, bool WIDE = false>
-__device__ __forceinline__ C weno5(C ae, C s0, C s1, C s2, C s3, C s4)
+
+// ---- FP32.  w = |e| s / 2: half the scaled value, so that the smoothness
+// terms need no factors (a quarter of a slope's square is the square of its
+// half; powers of two round nothing).
+struct WenoPoint32 {
+    float2 w, q;  // |e| s / 2, |e| s
+};
+struct WenoCurv32 {
+    float2 d, k;  // half the second difference, 13/3 of it
+};
+__device__ __forceinline__ WenoPoint32 weno_point(float2 s, const FaceArg<float> &g)
 {
-    const C q0 = xmul(ae, s0), q1 = xmul(ae, s1), q2 = xmul(ae, s2), q3 = xmul(ae, s3), q4 = xmul(ae, s4);
-    // second differences d_k and one-sided slopes l_k of the three stencils
-    const C d0 = xfma(kc<C>(-2), q1, xadd(q0, q2));
-    const C d1 = xfma(kc<C>(-2), q2, xadd(q1, q3));
-    const C d2 = xfma(kc<C>(-2), q3, xadd(q2, q4));
-    const C l0 = xfma(kc<C>(3), q2, xfma(kc<C>(-4), q1, q0));
-    const C l1 = xsub(q1, q3);
-    const C l2 = xfma(kc<C>(-4), q3, xfma(kc<C>(3), q2, q4));
+    const float2 w = xmul(g.aeh, s);
+    return WenoPoint32{w, xadd(w, w)};
+}
+__device__ __forceinline__ WenoCurv32 weno_curv(float2 w0, float2 w1, float2 w2)
+{
+    const float2 d = xfma(kc<float2>(-2), w1, xadd(w0, w2));
+    return WenoCurv32{d, xmul(make_float2(4.f * (float)(13.0 / 12.0), 4.f * (float)(13.0 / 12.0)), d)};
+}
+// the face from its five points and the curvatures at the middle three
+template <bool WIDE>
+__device__ __forceinline__ float2 weno_face(const WenoPoint32 &p0, const WenoPoint32 &p1, const WenoPoint32 &p2,
+                                            const WenoPoint32 &p3, const WenoPoint32 &p4, const WenoCurv32 &c0,
+                                            const WenoCurv32 &c1, const WenoCurv32 &c2)
+{
+    using V = float2;
+    // half the one-sided slopes of the three stencils
+    const V l0 = xfma(kc<V>(3), p2.w, xfma(kc<V>(-4), p1.w, p0.w));
+    const V l1 = xsub(p1.w, p3.w);
+    const V l2 = xfma(kc<V>(-4), p3.w, xfma(kc<V>(3), p2.w, p4.w));
     // eps + b_k
-    const C a0 = xfma(xmul(kc<C>(13.0 / 12.0), d0), d0, xfma(xmul(kc<C>(0.25), l0), l0, kc<C>(1e-6)));
-    const C a1 = xfma(xmul(kc<C>(13.0 / 12.0), d1), d1, xfma(xmul(kc<C>(0.25), l1), l1, kc<C>(1e-6)));
-    const C a2 = xfma(xmul(kc<C>(13.0 / 12.0), d2), d2, xfma(xmul(kc<C>(0.25), l2), l2, kc<C>(1e-6)));
-    C w0, w1, w2;
-    if (IsF32<C>::value && WIDE) {
-        const C m = xmin(a0, xmin(a1, a2));
-        const C s0 = face_div(m, a0), s1 = face_div(m, a1), s2 = face_div(m, a2);
-        w0 = xmul(kc<C>(0.1), xmul(s0, s0));
-        w1 = xmul(kc<C>(0.6), xmul(s1, s1));
-        w2 = xmul(kc<C>(0.3), xmul(s2, s2));
+    const V a0 = xfma(c0.k, c0.d, xfma(l0, l0, kc<V>(1e-6)));
+    const V a1 = xfma(c1.k, c1.d, xfma(l1, l1, kc<V>(1e-6)));
+    const V a2 = xfma(c2.k, c2.d, xfma(l2, l2, kc<V>(1e-6)));
+    V w0, w1, w2;  // weights, the middle one negative (its candidate is too)
+    if constexpr (WIDE) {
+        const V m = xmin(a0, xmin(a1, a2));
+        const V s0 = face_div(m, a0), s1 = face_div(m, a1), s2 = face_div(m, a2);
+        w0 = xmul(kc<V>(0.1), xmul(s0, s0));
+        w1 = xmul(kc<V>(-0.6), xmul(s1, s1));
+        w2 = xmul(kc<V>(0.3), xmul(s2, s2));
     } else {
-        const C p0 = xmul(a0, a0), p1 = xmul(a1, a1), p2 = xmul(a2, a2);
-        w0 = xmul(kc<C>(0.1), xmul(p1, p2));
-        w1 = xmul(kc<C>(0.6), xmul(p0, p2));
-        w2 = xmul(kc<C>(0.3), xmul(p0, p1));
+        const V b0 = xmul(a0, a0), b1 = xmul(a1, a1), b2 = xmul(a2, a2);
+        w0 = xmul(kc<V>(0.1), xmul(b1, b2));
+        w1 = xmul(kc<V>(-0.6), xmul(b0, b2));
+        w2 = xmul(kc<V>(0.3), xmul(b0, b1));
     }
-    // candidate reconstructions (times 6)
-    const C r0 = xfma(kc<C>(11), q2, xfma(kc<C>(-7), q1, xmul(kc<C>(2), q0)));
-    const C r1 = xfma(kc<C>(2), q3, xfma(kc<C>(5), q2, xneg(q1)));
-    const C r2 = xsub(xfma(kc<C>(5), q3, xmul(kc<C>(2), q2)), q4);
-    return face_div(xfma(w2, r2, xfma(w1, r1, xmul(w0, r0))), xmul(kc<C>(6), xadd(xadd(w0, w1), w2)));
+    // candidate reconstructions (times 3)
+    const V r0 = xfma(kc<V>(11), p2.w, xfma(kc<V>(-7), p1.w, p0.q));
+    const V r1 = xfma(kc<V>(-2), p3.w, xfma(kc<V>(-5), p2.w, p1.w));
+    const V r2 = xsub(xfma(kc<V>(5), p3.w, p2.q), p4.w);
+    return face_div(xfma(w2, r2, xfma(w1, r1, xmul(w0, r0))), xmul(kc<V>(3), xadd(xsub(w0, w1), w2)));
 }
-
-// the range-safe form out of line: the general paths that choose the form
-// at run time keep one inlined WENO5 (their code stays compact)
-template <class C>
-__device__ __noinline__ C weno5_wide(C ae, C s0, C s1, C s2, C s3, C s4)
+// NND (cpuLBM.cpp:1328-1356): c = |e| s1, the differences to |e| s2, |e| s0
+__device__ __forceinline__ float2 nnd_face(float2 s0, float2 s1, float2 s2, float2 c, const FaceArg<float> &g)
 {
-    return weno5<C, true>(ae, s0, s1, s2, s3, s4);
+    const float2 nae = make_float2(-g.ae.x, -g.ae.y);
+    const float2 nf = xfma(nae, s2, c), b = xfma(nae, s0, c);  // minus the forward difference, the backward one
+    return xfma(kc<float2>(0.5), make_float2(minmod(-nf.x, b.x), minmod(-nf.y, b.y)), c);
 }
 
-// WENO5 with the weight form of the sample
-template <class C>
-__device__ __forceinline__ C weno5_sp(const SampleParams &sp, C ae, C s0, C s1, C s2, C s3, C s4)
+// ---- FP64, on first differences e_j = s_{j+1} - s_j and second differences
+// d_k of the unscaled values: both schemes are homogeneous, so |e| can
+// multiply the flux difference once.  With the one-sided slopes m_k,
+//   eps + b_k = t_k + m_k^2,  t_k = 13/12 d_k^2 + eps,
+//   m0 = e1 + d0/2, m1 = e1 + d1/2, m2 = e2 - d2/2,
+// and the candidates are s + c_k/2, c0 = e1 + 2/3 d0, c1 = e1 + 2/3 d1,
+// c2 = e2 - d2/3 (weights 1, 6, 3): 29 operations a face in a line against
+// 39 for the form above, and the correction to the centre value is small
+// where the flow is smooth.
+__device__ __forceinline__ double2 weno_t(double2 d, double2 eps)
 {
-    if (sizeof(C) == 4 && sp.wide) return weno5_wide<C>(ae, s0, s1, s2, s3, s4);
-    return weno5<C, false>(ae, s0, s1, s2, s3, s4);
+    return xfma(xmul(kc<double2>(13.0 / 12.0), d), d, eps);
+}
+__device__ __forceinline__ double2 weno_face(double2 s, double2 e1, double2 e2, double2 d0, double2 d1, double2 d2,
+                                             double2 t0, double2 t1, double2 t2)
+{
+    using V = double2;
+    const V m0 = xfma(kc<V>(0.5), d0, e1), m1 = xfma(kc<V>(0.5), d1, e1), m2 = xfma(kc<V>(-0.5), d2, e2);
+    const V a0 = xfma(m0, m0, t0), a1 = xfma(m1, m1, t1), a2 = xfma(m2, m2, t2);
+    const V p0 = xmul(a0, a0), p1 = xmul(a1, a1), p2 = xmul(a2, a2), g = xmul(kc<V>(3.0), p0);
+    const V w0 = xmul(p1, p2), y = xmul(g, p2), w2 = xmul(g, p1);  // weights 1, 6 / 2, 3
+    const V c0 = xfma(kc<V>(2.0 / 3.0), d0, e1), c2 = xfma(kc<V>(-1.0 / 3.0), d2, e2);
+    const V c1 = xfma(kc<V>(4.0 / 3.0), d1, xadd(e1, e1));  // twice c1
+    const V num = xfma(y, c1, xfma(w2, c2, xmul(w0, c0)));
+    const V den = xfma(kc<V>(2.0), y, xadd(w0, w2));
+    return xfma(kc<V>(0.5), face_div(num, den), s);
+}
+__device__ __forceinline__ double2 nnd_face(double2 s1, double2 e0, double2 e1)
+{
+    return xfma(kc<double2>(0.5), make_double2(minmod(e1.x, e0.x), minmod(e1.y, e0.y)), s1);
 }
 
-// view of one sample's stage buffer and node flags
+// one face; FM: 0 NND, 1 WENO5, 2 WENO5 with the range-safe weights (FP32)
+template <int FM>
+__device__ __forceinline__ float2 face5(float2 s0, float2 s1, float2 s2, float2 s3, float2 s4, const FaceArg<float> &g)
+{
+    if constexpr (FM == 0) return nnd_face(s1, s2, s3, xmul(g.ae, s2), g);
+    else {
+        const WenoPoint32 p0 = weno_point(s0, g), p1 = weno_point(s1, g), p2 = weno_point(s2, g), p3 = weno_point(s3, g),
+                          p4 = weno_point(s4, g);
+        return weno_face<FM == 2>(p0, p1, p2, p3, p4, weno_curv(p0.w, p1.w, p2.w), weno_curv(p1.w, p2.w, p3.w),
+                                  weno_curv(p2.w, p3.w, p4.w));
+    }
+}
+template <int FM>
+__device__ __forceinline__ double2 face5(double2 s0, double2 s1, double2 s2, double2 s3, double2 s4,
+                                         const FaceArg<double> &g)
+{
+    const double2 e1 = xsub(s2, s1), e2 = xsub(s3, s2);
+    if constexpr (FM == 0) return nnd_face(s2, e1, e2);
+    else {
+        const double2 d0 = xsub(e1, xsub(s1, s0)), d1 = xsub(e2, e1), d2 = xsub(xsub(s4, s3), e2);
+        return weno_face(s2, e1, e2, d0, d1, d2, weno_t(d0, g.eps), weno_t(d1, g.eps), weno_t(d2, g.eps));
+    }
+}
+
+// the scheme read at run time (general tiles, wall factors); one compiled
+// copy of each scheme, out of line
+template <class C>
+__device__ __noinline__ Pair<C> face5_rt(int fm, Pair<C> s0, Pair<C> s1, Pair<C> s2, Pair<C> s3, Pair<C> s4,
+                                         FaceArg<C> g)
+{
+    if (fm == 0) return face5<0>(s0, s1, s2, s3, s4, g);
+    if constexpr (sizeof(C) == 4)
+        if (fm == 2) return face5<2>(s0, s1, s2, s3, s4, g);
+    return face5<1>(s0, s1, s2, s3, s4, g);
+}
+
+// flux differences along a line of LEN nodes: v[k] are the values at nodes
+// k - 3 in upwind order (k = 0 .. LEN + 4), out[n] = F(n) - F(n - 1) for the
+// nodes n = 0 .. LEN - 1, F(n) the face downwind of node n.  hook(n, F) may
+// replace the face (n = -1 .. LEN - 1; walls).
+template <int FM, int LEN, class HOOK>
+__device__ __forceinline__ void line_diffs(const float2 (&v)[LEN + 5], const FaceArg<float> &g, float2 (&out)[LEN],
+                                           HOOK hook)
+{
+    float2 prev;
+    if constexpr (FM == 0) {
+#pragma unroll
+        for (int n = -1; n < LEN; ++n) {
+            const float2 F = hook(n, nnd_face(v[n + 2], v[n + 3], v[n + 4], xmul(g.ae, v[n + 3]), g));
+            if (n >= 0) out[n] = xsub(F, prev);
+            prev = F;
+        }
+    } else {
+        WenoPoint32 p0 = weno_point(v[0], g), p1 = weno_point(v[1], g), p2 = weno_point(v[2], g),
+                    p3 = weno_point(v[3], g);
+        WenoCurv32 c0 = weno_curv(p0.w, p1.w, p2.w), c1 = weno_curv(p1.w, p2.w, p3.w);
+#pragma unroll
+        for (int n = -1; n < LEN; ++n) {
+            const WenoPoint32 p4 = weno_point(v[n + 5], g);
+            const WenoCurv32 c2 = weno_curv(p2.w, p3.w, p4.w);
+            const float2 F = hook(n, weno_face<FM == 2>(p0, p1, p2, p3, p4, c0, c1, c2));
+            if (n >= 0) out[n] = xsub(F, prev);
+            prev = F;
+            p0 = p1;
+            p1 = p2;
+            p2 = p3;
+            p3 = p4;
+            c0 = c1;
+            c1 = c2;
+        }
+    }
+}
+template <int FM, int LEN, class HOOK>
+__device__ __forceinline__ void line_diffs(const double2 (&v)[LEN + 5], const FaceArg<double> &g, double2 (&out)[LEN],
+                                           HOOK hook)
+{
+    using V = double2;
+    V prev;
+    if constexpr (FM == 0) {
+        V e0 = xsub(v[2], v[1]);
+#pragma unroll
+        for (int n = -1; n < LEN; ++n) {
+            const V e1 = xsub(v[n + 4], v[n + 3]);
+            const V F = hook(n, nnd_face(v[n + 3], e0, e1));
+            if (n >= 0) out[n] = xsub(F, prev);
+            prev = F;
+            e0 = e1;
+        }
+    } else {
+        V e1 = xsub(v[2], v[1]), e2 = xsub(v[3], v[2]);
+        V d0 = xsub(e1, xsub(v[1], v[0])), d1 = xsub(e2, e1);
+        V t0 = weno_t(d0, g.eps), t1 = weno_t(d1, g.eps);
+#pragma unroll
+        for (int n = -1; n < LEN; ++n) {
+            const V e3 = xsub(v[n + 5], v[n + 4]);
+            const V d2 = xsub(e3, e2);
+            const V t2 = weno_t(d2, g.eps);
+            const V F = hook(n, weno_face(v[n + 3], e1, e2, d0, d1, d2, t0, t1, t2));
+            if (n >= 0) out[n] = xsub(F, prev);
+            prev = F;
+            e1 = e2;
+            e2 = e3;
+            d0 = d1;
+            d1 = d2;
+            t0 = t1;
+            t1 = t2;
+        }
+    }
+}
+__device__ __forceinline__ int scheme_of(const SampleParams &sp) { return sp.fm ? (sp.wide ? 2 : 1) : 0; }
+
+// extrapolation over a solid edge (stencil): 2 f(m1) - f(m2)
+template <class V>
+__device__ __forceinline__ V extrapolate(V f1, V f2)
+{
+    return xsub(xadd(f1, f1), f2);
+}
+
 // One sample's stage buffer and node flags; offsets inside a sample fit in
-// 32 bits (26 planes of up to 2^26 nodes).
+// 32 bits (26 values of up to 2^26 nodes).
 template <class S>
 struct StageView {
     const S *__restrict__ st;        // plane 0 of the sample in the stage buffer
@@ -746,27 +969,27 @@ struct StageView {
     int pitch;
 };
 
+// the (f, h) pair of direction i at (x, y)
 template <class S>
-__device__ __forceinline__ S ldv(const StageView<S> &v, int p, int x, int y)
+__device__ __forceinline__ Pair<S> ldv(const StageView<S> &v, int i, int x, int y)
 {
-    return __ldg(v.st + (p * v.plane + y * v.pitch + x));
+    return __ldg(reinterpret_cast<const Pair<S> *>(v.st) + (i * v.plane + y * v.pitch + x));
 }
 
 // Exact stencil + reconstruction (stencil, cpuLBM.cpp:1171-1326, then NND/
-// WENO5) for the flux of plane p along `axis` at (x, y): boundary-aware
-// indices with reflections, and the linear extrapolation 2 f(m1) - f(m2)
-// over the first solid/fluid edge met by the stencil.
+// WENO5) for the flux (FP64: divided by |e|) of direction i along `axis` at
+// (x, y): boundary-aware indices with reflections, and the linear
+// extrapolation 2 f(m1) - f(m2) over the first solid/fluid edge met by the
+// stencil.
 template <class S, class C>
-__device__ __noinline__ C flux_exact(const SampleParams &sp, const StageView<S> &v, int x, int y, int p, int axis)
+__device__ __noinline__ Pair<C> flux_exact(const SampleParams &sp, const StageView<S> &v, int x, int y, int i, int axis)
 {
-    const int i = p < NQ ? p : p - NQ, pb = p - i;
-    const int e = axis == 0 ? isgn(c_EX[i]) : isgn(c_EY[i]);
-    if (e == 0) return C(0);
-    const C ae = (C)(sp.c * (double)abs(axis == 0 ? c_EX[i] : c_EY[i]));
-    const int L = sp.fm ? 5 : 3, low = (L - 1) / 2;
+    const int ev = axis == 0 ? c_EX[i] : c_EY[i];
+    const int e = isgn(ev);
+    const int L = sp.fm ? 5 : 3, low = (L - 1) / 2, j0 = 2 - low;  // NND: the middle three of five
     const int pos = axis == 0 ? x : y;
     const int j1 = pos - e * low;
-    C S5[5];
+    Pair<C> S5[5];
     int sld[5];
     int any = 0;
 #pragma unroll
@@ -774,9 +997,9 @@ __device__ __noinline__ C flux_exact(const SampleParams &sp, const StageView<S> 
         if (j < L) {
             int m;
             const int r = bc_index(sp, j1, e * j, axis, m);
-            const int pp = m ? pb + (axis == 0 ? c_MIR_EW[i] : c_MIR_NS[i]) : p;
+            const int ii = m ? (axis == 0 ? c_MIR_EW[i] : c_MIR_NS[i]) : i;
             const int xr = axis == 0 ? r : x, yr = axis == 0 ? y : r;
-            S5[j] = (C)ldv(v, pp, xr, yr);
+            S5[j] = ldv(v, ii, xr, yr);
             sld[j] = (v.nf[yr * v.pitch + xr] & NF_TYPE) == 2;
             any |= sld[j];
         }
@@ -790,75 +1013,83 @@ __device__ __noinline__ C flux_exact(const SampleParams &sp, const StageView<S> 
         }
         const int r1 = bc_index(sp, pe, e * diff, axis, m);
         const int r2 = bc_index(sp, pe, e * 2 * diff, axis, m);
-        const C v1 = axis == 0 ? (C)ldv(v, p, r1, y) : (C)ldv(v, p, x, r1);
-        const C v2 = axis == 0 ? (C)ldv(v, p, r2, y) : (C)ldv(v, p, x, r2);
-        const C ext = C(2) * v1 - v2;
+        const Pair<C> v1 = axis == 0 ? ldv(v, i, r1, y) : ldv(v, i, x, r1);
+        const Pair<C> v2 = axis == 0 ? ldv(v, i, r2, y) : ldv(v, i, x, r2);
+        const Pair<C> ext = extrapolate(v1, v2);
         // S5[jj] = ext; S5[jj - diff] = ext when inside the stencil
 #pragma unroll
         for (int j = 0; j < 5; ++j)
             if (j < L && (j == jj || (j == jj - diff))) S5[j] = ext;
     }
-    if (sp.fm) return weno5_sp<C>(sp, ae, S5[0], S5[1], S5[2], S5[3], S5[4]);
-    return nnd3<C>(ae, S5[0], S5[1], S5[2]);
+    const FaceArg<C> g = face_arg<C>(sp, ev);
+    if (j0) return face5_rt<C>(0, S5[0], S5[0], S5[1], S5[2], S5[2], g);
+    return face5_rt<C>(scheme_of(sp), S5[0], S5[1], S5[2], S5[3], S5[4], g);
 }
 
-// Stencil across a periodic edge with no solid in it: the five neighbours
-// with single periodic wrap, read from global memory.
+// Outgoing face flux (FP64: divided by |e|) of direction i along `axis` at a
+// non-solid node; nodes with no solid and no clamped or mirrored edge within
+// the stencil read the five neighbours directly (with single periodic wrap
+// across a periodic edge).
 template <class S, class C>
-__device__ __forceinline__ C flux_wrap(const SampleParams &sp, const StageView<S> &v, int x, int y, int p, int axis)
+__device__ __forceinline__ Pair<C> flux_axis(const SampleParams &sp, const StageView<S> &v, int x, int y, int i,
+                                             int axis, uint8_t nflag)
 {
-    const int i = p < NQ ? p : p - NQ;
     const int ev = axis == 0 ? c_EX[i] : c_EY[i];
-    if (ev == 0) return C(0);
+    const uint8_t slow = axis == 0 ? (NF_SOLX | NF_EDGX) : (NF_SOLY | NF_EDGY);
+    if (nflag & slow) return flux_exact<S, C>(sp, v, x, y, i, axis);
     const int e = ev > 0 ? 1 : -1;
-    const C ae = (C)(sp.c * (double)abs(ev));
-    const int N = axis == 0 ? sp.nx : sp.ny;
-    const int pos = axis == 0 ? x : y;
-    C q[5];
+    const bool wrap = (nflag & (axis == 0 ? NF_WRPX : NF_WRPY)) != 0;
+    const int N = axis == 0 ? sp.nx : sp.ny, pos = axis == 0 ? x : y;
+    Pair<C> q[5];
 #pragma unroll
     for (int j = 0; j < 5; ++j) {
         int r = pos + e * (j - 2);
-        r += r < 0 ? N : 0;
-        r -= r >= N ? N : 0;
-        q[j] = axis == 0 ? (C)ldv(v, p, r, y) : (C)ldv(v, p, x, r);
+        if (wrap) {
+            r += r < 0 ? N : 0;
+            r -= r >= N ? N : 0;
+        }
+        q[j] = axis == 0 ? ldv(v, i, r, y) : ldv(v, i, x, r);
     }
-    if (sp.fm) return weno5_sp<C>(sp, ae, q[0], q[1], q[2], q[3], q[4]);
-    return nnd3<C>(ae, q[1], q[2], q[3]);
-}
-
-// Outgoing face flux of plane p along `axis` at a non-solid node; the fast
-// path (no solid, no domain edge within the stencil) reads the five
-// neighbours directly.
-template <class S, class C>
-__device__ __forceinline__ C flux_axis(const SampleParams &sp, const StageView<S> &v, int x, int y, int p, int axis,
-                                       uint8_t nflag)
-{
-    const int i = p < NQ ? p : p - NQ;
-    const int ev = axis == 0 ? c_EX[i] : c_EY[i];
-    if (ev == 0) return C(0);
-    const uint8_t slow = axis == 0 ? (NF_SOLX | NF_EDGX) : (NF_SOLY | NF_EDGY);
-    if (nflag & slow) return flux_exact<S, C>(sp, v, x, y, p, axis);
-    if (nflag & (axis == 0 ? NF_WRPX : NF_WRPY)) return flux_wrap<S, C>(sp, v, x, y, p, axis);
-    const int e = ev > 0 ? 1 : -1;
-    const C ae = (C)(sp.c * (double)abs(ev));
-    const int stride = axis == 0 ? e : e * v.pitch;
-    const S *c0 = v.st + (p * v.plane + y * v.pitch + x);
-    if (sp.fm) {
-        return weno5_sp<C>(sp, ae, (C)__ldg(c0 - 2 * stride), (C)__ldg(c0 - stride), (C)__ldg(c0), (C)__ldg(c0 + stride),
-                        (C)__ldg(c0 + 2 * stride));
-    }
-    return nnd3<C>(ae, (C)__ldg(c0 - stride), (C)__ldg(c0), (C)__ldg(c0 + stride));
+    return face5_rt<C>(scheme_of(sp), q[0], q[1], q[2], q[3], q[4], face_arg<C>(sp, ev));
 }
 
 // wallFluxes (cpuLBM.cpp:1502-1590): for a solid node next to fluid,
 // alpha = (f flux of the fluid 4-neighbours into it) / (|e| f out of it),
 // weighted by the solid cell's 1/dx, 1/dy; one alpha for f and h.  Works on
 // full values (stored values + fr, the rest state of stored deviations) and
-// returns alpha - 1.
+// gives alpha - 1.  Sums in FP64, every operation explicitly rounded: the
+// stencil kernels form the factor of a straight wall themselves, with the
+// same bits.
 __constant__ int c_WXX[4] = {-1, 1, 0, 0};
 __constant__ int c_WYY[4] = {0, 0, -1, 1};
 __constant__ int c_WII[4][4] = {{1, 5, 8, 9}, {3, 6, 7, 11}, {2, 5, 6, 10}, {4, 7, 8, 12}};
 __constant__ int c_WINV[4][4] = {{3, 6, 7, 11}, {1, 5, 8, 9}, {4, 8, 7, 12}, {2, 6, 5, 10}};
+
+// sums of the fluxes in (F: a face flux, FP64's divided by |e|) and out
+// (v: a stored value), fr the rest value, ce = |e|, dd the cell width
+__device__ __forceinline__ double wall_in(double acc, float F, double fr, double ce, double dd)
+{
+    return __dadd_rn(acc, __ddiv_rn(__fma_rn(ce, fr, (double)F), dd));
+}
+__device__ __forceinline__ double wall_in(double acc, double F, double fr, double ce, double dd)
+{
+    return __dadd_rn(acc, __ddiv_rn(__dmul_rn(ce, __dadd_rn(F, fr)), dd));
+}
+__device__ __forceinline__ double wall_out(double acc, double v, double fr, double ce, double dd)
+{
+    return __dadd_rn(acc, __ddiv_rn(__dmul_rn(__dadd_rn(v, fr), ce), dd));
+}
+__device__ __forceinline__ double wall_ratio_m1(double fin, double fout) { return __dsub_rn(__ddiv_rn(fin, fout), 1.0); }
+
+// wallFluxes' alpha |e| f on full values, written for stored ones: |e| times
+// f_s + (alpha - 1)(f_s + f_ref), f and h (FP64: divided by |e|)
+template <class C>
+__device__ __forceinline__ Pair<C> wall_flux(C am1, Pair<C> fs, const double *fr, int i, const FaceArg<C> &g)
+{
+    const Pair<C> v = make_pair2(xfma(am1, xadd(fs.x, (C)fr[i]), fs.x), xfma(am1, xadd(fs.y, (C)fr[NQ + i]), fs.y));
+    if constexpr (sizeof(C) == 4) return xmul(g.ae, v);
+    else return v;
+}
 
 template <class S, class C>
 __device__ double wall_alpha_m1(const SampleParams &sp, const StageView<S> &v, int x, int y, double dxm, double dym,
@@ -875,14 +1106,13 @@ __device__ double wall_alpha_m1(const SampleParams &sp, const StageView<S> &v, i
         const double dd = axis == 0 ? dxm : dym;
         for (int q = 0; q < 4; ++q) {
             const int i = c_WII[j][q], io = c_WINV[j][q];
-            const double ai = sp.c * abs(axis == 0 ? c_EX[i] : c_EY[i]);
-            const double F = (double)flux_axis<S, C>(sp, v, xm, ym, i, axis, fl) + ai * fr[i];
-            fin += F / dd;
-            const double fo = (double)ldv(v, io, x, y) + fr[io];
-            fout += fo * (sp.c * abs(axis == 0 ? c_EX[io] : c_EY[io])) / dd;
+            const double ci = sp.c * abs(axis == 0 ? c_EX[i] : c_EY[i]);
+            const double co = sp.c * abs(axis == 0 ? c_EX[io] : c_EY[io]);
+            fin = wall_in(fin, flux_axis<S, C>(sp, v, xm, ym, i, axis, fl).x, fr[i], ci, dd);
+            fout = wall_out(fout, (double)ldv(v, io, x, y).x, fr[io], co, dd);
         }
     }
-    return fin / fout - 1.0;
+    return wall_ratio_m1(fin, fout);
 }
 
 }  // namespace uqlbm

@@ -7,6 +7,7 @@
 // Derived run parameters follow cpuLBM::refineInput / setupVars
 // (CODE/C++/VS2010/simLB/simLB/cpuLBM.cpp:283-450) and the step driver
 // follows runSimStep (main.cpp:32-112).
+#include "lbm_box.h"
 #include "lbm_common.h"
 #include "lbm_hdf5.h"
 #include "lbm_mat.h"
@@ -255,6 +256,10 @@ void prepare_sample(const HostSample &h, int prec, PreparedSample &out)
         for (double r : h.rho0) rho_max = std::max(rho_max, std::fabs(r));
         const double scale = 2.0 * h.c * rho_max * std::max(2.0, 10.0 * h.R * h.Tc);
         p.wide = (prec == LBM_PREC_F32 && !(scale <= 100.0)) ? 1 : 0;
+        // the FP64 reconstructions' epsilon, kept where its powers are normal
+        // numbers for any c (beyond these the weights are the linear ones, or
+        // epsilon does not matter)
+        p.eps1 = std::min(std::max(1e-6 / (h.c * h.c), 1e-35), 1e35);
     }
     // rest state of the stored deviations (FP32 path only)
     if (prec == LBM_PREC_F32) {
@@ -324,65 +329,101 @@ void prepare_sample(const HostSample &h, int prec, PreparedSample &out)
         }
 }
 
-// Tiles of one sample, each flagged simple when it and its 3-node halo lie
-// inside the domain and hold only plain fluid nodes.
-void cut_tiles(const uint8_t *flags, int pitch, int nx, int ny, int tx, int ty, int sflags, int gx, int sample,
-               std::vector<Tile> &out)
+// Tiles of one sample with their kinds.  A tile is a sweep tile when all
+// that its fluxes see (the tile and 3 nodes around it) is plain fluid or of
+// a form that fix_box (lbm_flux.cuh) completes: domain edges that wrap or
+// clamp, permanent nodes, and solids that are a straight wall, all of row 0
+// or row ny - 1 in the columns the tile sees (in rows of their own: 8 or
+// more rows, so that no stencil meets both walls).
+void cut_tiles(const uint8_t *flags, const SampleParams &p, int tx, int ty, int sample, std::vector<Tile> &out)
 {
-    const bool px = (sflags & SF_PERX) != 0, py = (sflags & SF_PERY) != 0;
+    const int nx = p.nx, ny = p.ny, pitch = p.pitch;
+    const bool px = (p.flags & SF_PERX) != 0, py = (p.flags & SF_PERY) != 0;
+    const int base = ((p.fm ? (p.wide ? 2 : 1) : 0) << TILE_FM_SHIFT) | (p.gx ? TILE_GHOST : 0);
+    // per row, the columns between which its permanent and solid nodes lie
+    // (most rows have none, and most tiles see no such row)
+    std::vector<int> lo(ny, nx), hi(ny, -1);
+    for (int y = 0; y < ny; ++y) {
+        const uint8_t *row = flags + (long long)y * pitch;
+        for (int x = 0; x < nx; ++x)
+            if (row[x] & NF_TYPE) {
+                lo[y] = std::min(lo[y], x);
+                hi[y] = x;
+            }
+    }
     for (int y0 = 0; y0 < ny; y0 += ty)
         for (int x0 = 0; x0 < nx; x0 += tx) {
-            int gid = (int)out.size();
-            const bool in_x = x0 >= 3 && x0 + tx + 3 <= nx, in_y = y0 >= 3 && y0 + ty + 3 <= ny;
-            if (in_x && in_y) {
-                bool simple = true;
-                for (int y = y0 - 3; y < y0 + ty + 3 && simple; ++y)
-                    for (int x = x0 - 3; x < x0 + tx + 3; ++x)
-                        if (flags[(long long)y * pitch + x] != 0) { simple = false; break; }
-                if (simple) gid |= TILE_SIMPLE;
-            } else if ((in_x || px) && (in_y || py) && x0 + tx <= nx && y0 + ty <= ny) {
-                // a full tile whose halo crosses a periodic edge: plain fluid
-                // everywhere in the halo (periodic images included), and no
-                // flag but the stencil-wraps bits
-                bool wrap = true;
-                for (int y = y0 - 3; y < y0 + ty + 3 && wrap; ++y)
-                    for (int x = x0 - 3; x < x0 + tx + 3; ++x) {
-                        const int xw = ((x % nx) + nx) % nx, yw = ((y % ny) + ny) % ny;
-                        if (flags[(long long)yw * pitch + xw] & ~(NF_WRPX | NF_WRPY)) { wrap = false; break; }
+            Tile t{sample, x0, y0, (int)out.size(), base, {0, 0, 0}};
+            const int xe = std::min(x0 + tx, nx), ye = std::min(y0 + ty, ny);  // the tile's nodes
+            const bool w = x0 < 3, e = x0 + tx + 3 > nx, s = y0 < 3, n = y0 + ty + 3 > ny;
+            bool fixed = false;  // permanent nodes in the tile, or solids in sight
+            bool sweep = true, fix = ((w || e) && !p.gx) || s || n;
+            if (!px && ((w && (p.flags & SF_MIRW)) || (e && (p.flags & SF_MIRE)))) sweep = false;
+            if (!py && ((s && (p.flags & SF_MIRS)) || (n && (p.flags & SF_MIRN)))) sweep = false;
+            // solids seen in row 0, in row ny - 1 and elsewhere; other nodes seen in those rows
+            bool s0 = false, s1 = false, f0 = false, f1 = false;
+            const int xa = x0 - 3, xb = xe + 3;  // columns in sight: [xa, xb)
+            for (int yy = y0 - 3; yy < ye + 3 && sweep; ++yy) {
+                if (!py && (yy < 0 || yy >= ny)) continue;
+                const int y = py ? ((yy % ny) + ny) % ny : yy;
+                if (hi[y] < 0 || ((xa >= 0 && xb <= nx) && (hi[y] < xa || lo[y] >= xb))) {
+                    f0 = f0 || y == 0;
+                    f1 = f1 || y == ny - 1;
+                    continue;
+                }
+                const uint8_t *row = flags + (long long)y * pitch;
+                for (int xx = xa; xx < xb; ++xx) {
+                    if (!px && (xx < 0 || xx >= nx)) continue;
+                    const int type = row[xx >= 0 && xx < nx ? xx : ((xx % nx) + nx) % nx] & NF_TYPE;
+                    if (type != 2) {
+                        if (y == 0) f0 = true;
+                        if (y == ny - 1) f1 = true;
+                        if (type && xx >= x0 && xx < xe && yy >= y0 && yy < ye) fixed = true;
+                        continue;
                     }
-                // crossing only the x edges of a sample with ghost columns,
-                // the staged box needs nothing more: a simple tile
-                if (wrap) gid |= gx && in_y ? TILE_SIMPLE : TILE_WRAP;
+                    fixed = true;
+                    if (y == 0) s0 = true;
+                    else if (y == ny - 1) s1 = true;
+                    else { sweep = false; break; }
+                }
             }
-            out.push_back(Tile{sample, x0, y0, gid});
+            fix = fix || fixed;
+            if ((s0 && f0) || (s1 && f1) || ((s0 || s1) && (py || ny < 8))) sweep = false;
+            if (sweep) {
+                // completed by periodic images alone
+                const bool wraps = fix && !fixed && ((!w && !e) || px) && ((!s && !n) || py);
+                t.kind |= TILE_SWEEP | (fix ? TILE_FIX : 0) | (s0 ? TILE_WALLS : 0) | (s1 ? TILE_WALLN : 0) |
+                          (wraps ? TILE_WRAP : 0);
+            }
+            out.push_back(t);
         }
 }
 
-// TMA descriptors of a sample, each over the 26 planes as a 3D tensor
-// (x, y, plane): stage buffers 2 and 3 with the flux kernels' staged halo
-// box (one plane), and the state with the tile's own nodes over
-// PREFETCH_PLANES planes (the update's reads of f or of h).
-void encode_stage_maps(int prec, const SampleParams &p, unsigned char *state, unsigned char *buf2,
-                       unsigned char *buf3, int tx, int ty, CUtensorMap *maps)
+void needed_walls(const SampleParams &p, int tx, int ty, const Tile *tiles, const std::vector<WallNode> &walls,
+                  std::vector<WallNode> &out)
+{
+    out.clear();
+    const int ntx = (p.nx + tx - 1) / tx;
+    auto general = [&](int x, int y) {
+        x = (p.flags & SF_PERX) ? (x + p.nx) % p.nx : std::min(std::max(x, 0), p.nx - 1);
+        y = (p.flags & SF_PERY) ? (y + p.ny) % p.ny : std::min(std::max(y, 0), p.ny - 1);
+        return !tile_sweep(tiles[(y / ty) * ntx + x / tx]);
+    };
+    for (const WallNode &w : walls)
+        if (general(w.x, w.y) || general(w.x - 1, w.y) || general(w.x + 1, w.y) || general(w.x, w.y - 1) ||
+            general(w.x, w.y + 1))
+            out.push_back(w);
+}
+
+// TMA descriptors of a sample: stage buffers 2 and 3 over the 13 planes of
+// pairs, each with the stencil kernels' three box shapes (encode_box_map).
+void encode_stage_maps(int prec, const SampleParams &p, unsigned char *buf2, unsigned char *buf3, int tx, int ty,
+                       CUtensorMap *maps)
 {
     auto enc = tensor_map_encoder();
-    const size_t es = prec == LBM_PREC_F64 ? 8 : 4;
-    for (int b = 0; b < MAPS_PER_SAMPLE; ++b) {
-        // with ghost columns the tensor starts at the left ghosts and spans
-        // the pitch (boxes at the x edges then read the images); else it is
-        // the domain and boxes read zeros beyond it
-        unsigned char *base = (b == 0 ? buf2 : b == 1 ? buf3 : state) + (size_t)(p.state_off - p.gx) * es;
-        cuuint64_t dims[3] = {(cuuint64_t)(p.gx ? p.pitch : p.nx), (cuuint64_t)p.ny, (cuuint64_t)NPL};
-        cuuint64_t strides[2] = {(cuuint64_t)p.pitch * es, (cuuint64_t)p.plane * es};
-        cuuint32_t halo[3] = {(cuuint32_t)(tx + 8), (cuuint32_t)(ty + 6), 1};
-        cuuint32_t own[3] = {(cuuint32_t)tx, (cuuint32_t)ty, (cuuint32_t)PREFETCH_PLANES};
-        cuuint32_t estr[3] = {1, 1, 1};
-        CUresult r = enc(&maps[b], prec == LBM_PREC_F64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                         3, base, dims, strides, b < 2 ? halo : own, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) throw LbmError(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-    }
+    for (int b = 0; b < MAPS_PER_SAMPLE; ++b)
+        if (!encode_box_map(enc, prec == LBM_PREC_F64, p, b < 3 ? buf2 : buf3, b % 3, tx, ty, &maps[b]))
+            throw LbmError(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
 }
 
 }  // namespace uqlbm
@@ -403,9 +444,11 @@ struct lbm_batch {
     std::vector<SampleParams> sp;
     std::vector<Tile> tiles_all, tiles_rk3;
     std::vector<Tile> tiles_by_rk[4], tiles_flux[4];  // by RKMETHOD: sample order; by kind
-    // leading simple tiles and the wrap tiles after them in tiles_flux, tiles_rk3
-    int ns_by_rk[4] = {0, 0, 0, 0}, nw_by_rk[4] = {0, 0, 0, 0}, ns_rk3 = 0, nw_rk3 = 0;
-    std::vector<WallNode> walls_all, walls_rk3;
+    // leading sweep tiles in tiles_flux, tiles_rk3
+    int ns_by_rk[4] = {0, 0, 0, 0}, ns_rk3 = 0, kinds[4][2] = {}, kinds_rk3[2] = {};
+    std::vector<std::vector<WallNode>> walls_of;  // by sample: solid nodes next to fluid
+    std::vector<WallNode> walls_all, walls_rk3;   // those the current tiles need
+    std::vector<WallNode> every_wall, every_wall_rk3;
     std::vector<int> tile_first, tile_count;
     long long total_state = 0, total_nodes = 0, lattice_nodes = 0;
     size_t max_nodes = 0;
@@ -418,7 +461,7 @@ struct lbm_batch {
     DevBuf<SampleParams> d_sp;
     DevBuf<Tile> d_tiles_all, d_tiles_rk3;
     DevBuf<Tile> d_tiles_by_rk[4], d_tiles_flux[4];
-    DevBuf<WallNode> d_walls_all, d_walls_rk3;
+    DevBuf<WallNode> d_walls_all, d_walls_rk3, d_every_wall, d_every_wall_rk3;
     DevBuf<CUtensorMap> d_maps;
     DevBuf<double> d_fref;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [want_residual]
@@ -435,8 +478,7 @@ struct lbm_batch {
     }
 
     // Tile lists for the current tile shape: every sample cut into tx x ty
-    // tiles, each flagged simple when it and its 3-node halo lie inside the
-    // domain and hold only plain fluid nodes.
+    // tiles of their kinds, and the wall nodes that the general ones need.
     void make_tiles()
     {
         tiles_all.clear();
@@ -444,12 +486,18 @@ struct lbm_batch {
         for (auto &v : tiles_by_rk) v.clear();
         tile_first.clear();
         tile_count.clear();
+        walls_all.clear();
+        walls_rk3.clear();
+        std::vector<WallNode> need;
         for (size_t k = 0; k < hs.size(); ++k) {
             const HostSample &h = hs[k];
             SampleParams &p = sp[k];
             p.first_tile = (int)tiles_all.size();
-            cut_tiles(flags_host.data() + p.node_off, p.pitch, h.nx, h.ny, tx, ty, p.flags, p.gx, (int)k, tiles_all);
+            cut_tiles(flags_host.data() + p.node_off, p, tx, ty, (int)k, tiles_all);
             p.ntile = (int)tiles_all.size() - p.first_tile;
+            needed_walls(p, tx, ty, tiles_all.data() + p.first_tile, walls_of[k], need);
+            walls_all.insert(walls_all.end(), need.begin(), need.end());
+            if (h.rk == 1) walls_rk3.insert(walls_rk3.end(), need.begin(), need.end());
             for (int t = p.first_tile; t < p.first_tile + p.ntile; ++t) {
                 tiles_by_rk[h.rk].push_back(tiles_all[t]);
                 if (h.rk == 1) tiles_rk3.push_back(tiles_all[t]);
@@ -461,9 +509,9 @@ struct lbm_batch {
         // the pointwise phase keeps the sample order
         for (int m = 0; m < 4; ++m) {
             tiles_flux[m] = tiles_by_rk[m];
-            order_by_kind(tiles_flux[m], ns_by_rk[m], nw_by_rk[m]);
+            order_by_kind(tiles_flux[m], ns_by_rk[m], kinds[m]);
         }
-        order_by_kind(tiles_rk3, ns_rk3, nw_rk3);
+        order_by_kind(tiles_rk3, ns_rk3, kinds_rk3);
     }
 
     void upload_tiles()
@@ -475,19 +523,20 @@ struct lbm_batch {
             d_tiles_by_rk[m].upload(tiles_by_rk[m], stream);
             d_tiles_flux[m].upload(tiles_flux[m], stream);
         }
+        d_walls_all.upload(walls_all, stream);
+        d_walls_rk3.upload(walls_rk3, stream);
         d_tile_first.upload(tile_first, stream);
         d_tile_count.upload(tile_count, stream);
         partial.alloc(tiles_all.size());
     }
 
-    // TMA descriptors: per sample and stage buffer, the 26 planes as a 3D
-    // tensor (x, y, plane) with the staged halo box of the flux kernels
+    // TMA descriptors of every sample
     void make_maps()
     {
         const int n = (int)hs.size();
         std::vector<CUtensorMap> maps(MAPS_PER_SAMPLE * n);
         for (int k = 0; k < n; ++k)
-            encode_stage_maps(prec, sp[k], state.p, buf2.p, buf3.p, tx, ty, &maps[MAPS_PER_SAMPLE * k]);
+            encode_stage_maps(prec, sp[k], buf2.p, buf3.p, tx, ty, &maps[MAPS_PER_SAMPLE * k]);
         d_maps.upload(maps, stream);
     }
 
@@ -611,11 +660,10 @@ struct lbm_batch {
             v_dx.insert(v_dx.end(), ps.dx.begin(), ps.dx.end());
             v_dy.insert(v_dy.end(), ps.dy.begin(), ps.dy.end());
             flags.insert(flags.end(), ps.flags.begin(), ps.flags.end());
-            for (WallNode w : ps.walls) {
-                w.sample = k;
-                walls_all.push_back(w);
-                if (h.rk == 1) walls_rk3.push_back(w);
-            }
+            for (WallNode &w : ps.walls) w.sample = k;
+            walls_of.push_back(ps.walls);
+            every_wall.insert(every_wall.end(), ps.walls.begin(), ps.walls.end());
+            if (h.rk == 1) every_wall_rk3.insert(every_wall_rk3.end(), ps.walls.begin(), ps.walls.end());
             state_off += NPL * p.plane + (p.gx ? GHOST_SLACK : 0);
             node_off += p.plane;
             lattice_nodes += (long long)h.nx * h.ny;
@@ -648,8 +696,8 @@ struct lbm_batch {
         dyv.upload(v_dy, stream);
         d_fref.upload(fref_host, stream);
         upload_tiles();
-        d_walls_all.upload(walls_all, stream);
-        d_walls_rk3.upload(walls_rk3, stream);
+        d_every_wall.upload(every_wall, stream);
+        d_every_wall_rk3.upload(every_wall_rk3, stream);
         scratch.alloc(std::max<size_t>(5 * max_nodes, 2 * 13 * max_nodes));
         host_status.assign(n, 0);
         host_residual.assign(n, 1.0);
@@ -692,11 +740,15 @@ struct lbm_batch {
         StepLists l;
         for (int m = 0; m < 4; ++m) {
             l.pointwise[m] = TileRun{d_tiles_by_rk[m].p, (int)tiles_by_rk[m].size()};
-            split_runs(d_tiles_flux[m].p, (int)tiles_flux[m].size(), ns_by_rk[m], nw_by_rk[m], l.simple[m], l.wrap[m],
-                       l.general[m]);
+            split_runs(d_tiles_flux[m].p, (int)tiles_flux[m].size(), ns_by_rk[m], l.sweep[m], l.general[m]);
         }
-        if (any_rk3)
-            split_runs(d_tiles_rk3.p, (int)tiles_rk3.size(), ns_rk3, nw_rk3, l.rk3_simple, l.rk3_wrap, l.rk3_general);
+        if (any_rk3) split_runs(d_tiles_rk3.p, (int)tiles_rk3.size(), ns_rk3, l.rk3_sweep, l.rk3_general);
+        std::copy(&kinds[0][0], &kinds[0][0] + 8, &l.kinds[0][0]);
+        std::copy(kinds_rk3, kinds_rk3 + 2, l.rk3_kinds);
+        l.every_wall = d_every_wall.p;
+        l.n_every_wall = (int)every_wall.size();
+        l.every_wall_rk3 = d_every_wall_rk3.p;
+        l.n_every_wall_rk3 = (int)every_wall_rk3.size();
         l.samples = d_sp.p;
         l.nsamples = (int)hs.size();
         l.any_ghost = any_ghost;
@@ -707,19 +759,21 @@ struct lbm_batch {
         return l;
     }
 
-    // One step.  ev (optional) receives 7 events around the phases:
-    // [0] start, then after pointwise, walls 2, phase 1, walls 3, phase 2,
-    // residual.
+    // One step, phase by phase or not.  ev (optional, phased only) receives
+    // 7 events around the phases: [0] start, then after pointwise, walls 2,
+    // phase 1, walls 3, phase 2, residual.
     template <class S, class C>
-    void enqueue_step_t(int want_res, cudaEvent_t *ev = nullptr)
+    void enqueue_step_t(int want_res, bool phased, cudaEvent_t *ev = nullptr)
     {
-        enqueue_step_phases<S, C>(args<S>(want_res), lists(), stream, ev);
+        if (phased) enqueue_step_phased<S, C>(args<S>(want_res), lists(), stream, ev);
+        else uqlbm::enqueue_step<S, C>(args<S>(want_res), lists(), stream);
         if (want_res)
             CU(launch_residual(d_sp.p, (int)hs.size(), partial.p, d_tile_first.p, d_tile_count.p, residual.p, stream));
         if (ev) CU(cudaEventRecord(ev[6], stream));
     }
 
-    int launches_per_step(int want_res) const { return step_launches(lists()) + (want_res ? 1 : 0); }
+    int launches_per_step(int want_res) const { return phased_launches(lists()) + (want_res ? 1 : 0); }
+    int graph_launches(int want_res) const { return step_launches(lists()) + (want_res ? 1 : 0); }
 
     void profile(int n, double *ms, int nph)
     {
@@ -727,8 +781,8 @@ struct lbm_batch {
         for (auto &e : ev) CU(cudaEventCreate(&e));
         std::vector<double> acc(6, 0.0);
         for (int k = 0; k < n; ++k) {
-            if (prec == LBM_PREC_F64) enqueue_step_t<double, double>(1, ev);
-            else enqueue_step_t<float, float>(1, ev);
+            if (prec == LBM_PREC_F64) enqueue_step_t<double, double>(1, true, ev);
+            else enqueue_step_t<float, float>(1, true, ev);
             CU(cudaEventSynchronize(ev[6]));
             for (int p = 0; p < 6; ++p) {
                 float t = 0;
@@ -831,8 +885,8 @@ struct lbm_batch {
 
     void enqueue_step(int want_res)
     {
-        if (prec == LBM_PREC_F64) enqueue_step_t<double, double>(want_res);
-        else enqueue_step_t<float, float>(want_res);
+        if (prec == LBM_PREC_F64) enqueue_step_t<double, double>(want_res, !use_graph);
+        else enqueue_step_t<float, float>(want_res, !use_graph);
     }
 
     void launch_steps(int n, int want_res)
@@ -1313,6 +1367,8 @@ lbm_status lbm_batch_autotune(lbm_batch *b, const int *candidates, int n_candida
 }
 
 int lbm_batch_launches_per_step(lbm_batch *b, int want_residual) { return b ? b->launches_per_step(want_residual) : 0; }
+
+int lbm_batch_graph_launches(lbm_batch *b, int want_residual) { return b ? b->graph_launches(want_residual) : 0; }
 
 lbm_status lbm_batch_set_dist(lbm_batch *b, int sample, const double *f, const double *hh)
 {

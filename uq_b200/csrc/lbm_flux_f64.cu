@@ -1,0 +1,8 @@
+// The FP64 instances of the stencil kernels (a translation unit of their own:
+// the build compiles the two precisions side by side).
+#include "lbm_flux.cuh"
+
+namespace uqlbm {
+template cudaError_t launch_flux<double>(int, const KArgs<double> &, int, int, cudaStream_t);
+template cudaError_t prepare_flux<double>();
+}  // namespace uqlbm

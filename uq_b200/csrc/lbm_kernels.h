@@ -16,16 +16,13 @@ constexpr int STATUS_EQ = 1;         // equilibrium mass check (cpuLBM.cpp:839-8
 constexpr int STATUS_NONFINITE = 2;  // NaN / Inf / rho <= 0 in the state
 constexpr int STATUS_TIMEOUT = 4;    // a bounded device-side wait ran out
 
-// tensor maps per sample: the stage buffers 2 and 3 with the stencil
-// kernels' halo box, and the state with a box of the tile's own nodes over
-// 13 planes (the f or the h half of the state, prefetched for the update)
-constexpr int MAPS_PER_SAMPLE = 3;
-constexpr int PREFETCH_PLANES = 13;
+// tensor maps per sample: the stage buffers 2 and 3, each with the stencil
+// kernels' three box shapes (x lines, y lines, both; see lbm_flux.cuh)
+constexpr int MAPS_PER_SAMPLE = 6;
 // the default tile shape, also compiled into the stencil kernels (box
-// widths, strides and the thread-to-node map become constants); other shapes
-// run the same kernels with the shape read at run time.  A tile row of 32 is
-// one warp: a row's x neighbours sit in the same warp and its staged-box
-// reads are unit-stride across the warp.
+// widths, strides and the thread-to-line map become constants); other shapes
+// run kernels with the shape read at run time.  Of a 32 x 8 tile, the lines
+// of one direction along either axis are one warp's work (see lbm_flux.cuh).
 constexpr int TILE_CX = 32, TILE_CY = 8;
 
 struct WallNode {
@@ -48,9 +45,14 @@ struct KArgs {
     double *partial;  // per-tile residual partial sums
     int *status;      // per-sample status bits
     const double *tdx, *tdy, *dxv, *dyv;
-    const CUtensorMap *tmaps;  // per sample MAPS_PER_SAMPLE maps: [buffer 2, buffer 3, state]
+    const CUtensorMap *tmaps;  // per sample MAPS_PER_SAMPLE maps: [buffer 2, buffer 3][box shape]
+    int slots;                 // boxes resident at a time (other tile shapes)
     const double *fref;        // per sample: 26 rest-state values subtracted from the stored state
     int want_residual;
+    // phases launched apart (enqueue_step_phased): the pointwise kernel leaves
+    // the ghost columns to k_fill_ghosts, and straight walls take their
+    // factors from k_wall
+    int phased;
     double eq_tol;
 #ifdef __CUDACC__
     // alpha is stored in the compute type of the kernel instantiation
@@ -59,18 +61,20 @@ struct KArgs {
 #endif
 };
 
-// Which tiles a stencil-phase launch covers: FLUX_SIMPLE, FLUX_WRAP and
-// FLUX_GENERAL run the kernel compiled for that kind alone over a list
-// holding only that kind; FLUX_BOTH runs the simple and the general kernel
-// over a list of those two kinds (each skips the other kind's tiles).
-enum FluxPath { FLUX_BOTH = 0, FLUX_SIMPLE = 1, FLUX_GENERAL = 2, FLUX_WRAP = 3 };
+// Which tiles a stencil-phase launch covers: the sweep tiles or the general
+// tiles of its list, one kernel each (see TILE_SWEEP).
+enum FluxPath { FLUX_SWEEP = 1, FLUX_GENERAL = 2 };
 
 template <class S, class C>
 cudaError_t launch_phase(const KArgs<S> &a, int phase, int rk, const Tile *tiles, int ntiles, const WallNode *walls,
-                         int nwalls, cudaStream_t st, int path = FLUX_BOTH);
+                         int nwalls, cudaStream_t st, int path = FLUX_GENERAL);
 template <class S, class C>
 cudaError_t prepare_kernels();
-size_t flux_smem_bytes(int prec, int tx, int ty);
+// the stencil kernels (lbm_flux_f32.cu, lbm_flux_f64.cu); mode as k_flux's
+template <class S>
+cudaError_t launch_flux(int mode, const KArgs<S> &a, int ntiles, int path, cudaStream_t st);
+template <class S>
+cudaError_t prepare_flux();
 template <class S>
 cudaError_t launch_init(const KArgs<S> &a, const double *rho, const double *ux, const double *uy, const double *T,
                         cudaStream_t st);

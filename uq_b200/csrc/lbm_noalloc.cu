@@ -11,6 +11,8 @@
 // The array is reserved on every GPU that loads this library, until the
 // process exits.  Every call shares it and overwrites what the last call
 // left; calls that overlap on the GPU (two streams, two threads) race on it.
+#include "lbm_box.h"
+#include "lbm_common.h"
 #include "lbm_device.cuh"
 #include "lbm_host.h"
 #include "lbm_kernels.h"
@@ -19,8 +21,10 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <vector>
 
 namespace uqlbm {
 
@@ -44,12 +48,12 @@ constexpr size_t NA_OFF_SP = NA_OFF_TILES + na_align(NA_MAX_TILES * sizeof(Tile)
 constexpr size_t NA_OFF_STATUS = NA_OFF_SP + na_align(sizeof(SampleParams));
 constexpr size_t NA_OFF_FREF = NA_OFF_STATUS + na_align(sizeof(int));
 constexpr size_t NA_OFF_MAPS = NA_OFF_FREF + na_align(NPL * sizeof(double));
-constexpr size_t NA_BYTES = NA_OFF_MAPS + na_align(2 * sizeof(CUtensorMap));
+constexpr size_t NA_BYTES = NA_OFF_MAPS + na_align(MAPS_PER_SAMPLE * sizeof(CUtensorMap));
 
 // the scratch: reserved per device by loading the module, never cudaMalloc'd
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
 
-// node flags (as the engine computes them on the host), tile list, spacing
+// node flags (as the engine computes them on the host), spacing
 // tables and cleared status / wall factors / rest state
 __global__ void k_na_setup(int nx, int ny, int pitch, int flags, double dx, double dy, double dt, unsigned char *base)
 {
@@ -85,10 +89,6 @@ __global__ void k_na_setup(int nx, int ny, int pitch, int flags, double dx, doub
         lines[2 * NA_MAX_LINE + k] = dx;
         lines[3 * NA_MAX_LINE + k] = dy;
     }
-    const int tiles_x = (nx + NA_TX - 1) / NA_TX, tiles_y = (ny + NA_TY - 1) / NA_TY;
-    Tile *tiles = reinterpret_cast<Tile *>(base + NA_OFF_TILES);
-    for (long long t = tid; t < (long long)tiles_x * tiles_y; t += (long long)gridDim.x * blockDim.x)
-        tiles[t] = Tile{0, (int)(t % tiles_x) * NA_TX, (int)(t / tiles_x) * NA_TY, (int)t};
     double *fref = reinterpret_cast<double *>(base + NA_OFF_FREF);
     if (tid < NPL) fref[tid] = 0.0;  // the FP64 path stores f and h in full
     if (tid == 0) *reinterpret_cast<int *>(base + NA_OFF_STATUS) = 0;
@@ -98,9 +98,9 @@ __global__ void k_na_setup(int nx, int ny, int pitch, int flags, double dx, doub
 // also seed the stage buffers
 __global__ void k_na_io(int nx, int ny, int pitch, double *f, double *h, unsigned char *base, int to_caller)
 {
-    double *st = reinterpret_cast<double *>(base + NA_OFF_STATE);
-    double *b2 = reinterpret_cast<double *>(base + NA_OFF_BUF2);
-    double *b3 = reinterpret_cast<double *>(base + NA_OFF_BUF3);
+    double2 *st = reinterpret_cast<double2 *>(base + NA_OFF_STATE);
+    double2 *b2 = reinterpret_cast<double2 *>(base + NA_OFF_BUF2);
+    double2 *b3 = reinterpret_cast<double2 *>(base + NA_OFF_BUF3);
     const uint8_t *nf = base + NA_OFF_FLAGS;
     const long long plane = (long long)ny * pitch;
     const long long n = (long long)nx * ny * NQ;
@@ -108,17 +108,17 @@ __global__ void k_na_io(int nx, int ny, int pitch, double *f, double *h, unsigne
         const int i = (int)(k % NQ);
         const long long xy = k / NQ;
         const int y = (int)(xy % ny), x = (int)(xy / ny);
-        const long long o = (long long)y * pitch + x;
-        const long long of = i * plane + o, oh = (NQ + i) * plane + o;
+        const long long o = (long long)y * pitch + x, e = i * plane + o;
         if (to_caller) {
-            f[k] = st[of];
-            h[k] = st[oh];
+            const double2 v = st[e];
+            f[k] = v.x;
+            h[k] = v.y;
         } else {
-            st[of] = f[k];
-            st[oh] = h[k];
+            const double2 v = make_double2(f[k], h[k]);
+            st[e] = v;
             if (nf[o] & NF_TYPE) {
-                b2[of] = f[k]; b3[of] = f[k];
-                b2[oh] = h[k]; b3[oh] = h[k];
+                b2[e] = v;
+                b3[e] = v;
             }
         }
     }
@@ -218,8 +218,6 @@ static lbm_status step_noalloc(const lbm_config *cfg, int Nx, int Ny, const int 
     sp.flags = sc.flags;
     sp.rk = sc.rk;
     sp.fm = sc.fm;
-    const int tiles_x = (Nx + NA_TX - 1) / NA_TX, tiles_y = (Ny + NA_TY - 1) / NA_TY;
-    sp.ntile = tiles_x * tiles_y;
     sp.plane = (long long)Ny * pitch;
     sp.R = sc.R;
     sp.bR = sc.b * sc.R;
@@ -232,6 +230,7 @@ static lbm_status step_noalloc(const lbm_config *cfg, int Nx, int Ny, const int 
     sp.dt = sc.dt;
     sp.c = sc.c;
     sp.inv_mu = 1.0 / sc.mu;
+    sp.eps1 = std::min(std::max(1e-6 / (sc.c * sc.c), 1e-35), 1e35);
     sp.two_over_bR = 2.0 / (sc.b * sc.R);
     sp.visc = sc.mu_model;
     sp.visc_exp = sc.mu_model == 1 ? 0.5 + sc.upsilon : 1.5;
@@ -241,21 +240,26 @@ static lbm_status step_noalloc(const lbm_config *cfg, int Nx, int Ny, const int 
     sp.T0n = 1.0;
     sp.shref = 0.0;
 
-    CUtensorMap maps[2];
-    for (int b = 0; b < 2; ++b) {
-        cuuint64_t dims[3] = {(cuuint64_t)Nx, (cuuint64_t)Ny, (cuuint64_t)NPL};
-        cuuint64_t strides[2] = {(cuuint64_t)pitch * sizeof(double), (cuuint64_t)sp.plane * sizeof(double)};
-        cuuint32_t box[3] = {(cuuint32_t)(NA_TX + 8), (cuuint32_t)(NA_TY + 6), 1};
-        cuuint32_t estr[3] = {1, 1, 1};
-        if (encoder()(&maps[b], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, base + (b == 0 ? NA_OFF_BUF2 : NA_OFF_BUF3), dims,
-                      strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    // the tiles and their kinds, from the cell types in pitch layout
+    std::vector<uint8_t> types((size_t)sp.plane, 0);
+    for (int x = 0; x < Nx; ++x)
+        for (int y = 0; y < Ny; ++y) types[(size_t)y * pitch + x] = (uint8_t)cellType[(size_t)x * Ny + y];
+    std::vector<Tile> tiles;
+    cut_tiles(types.data(), sp, NA_TX, NA_TY, 0, tiles);
+    int ns = 0;
+    order_by_kind(tiles, ns);
+    if ((int)tiles.size() > NA_MAX_TILES) throw LbmError(LBM_ERR_INVALID, "domain exceeds lbm_step_noalloc's tile list");
+    sp.ntile = (int)tiles.size();
+
+    CUtensorMap maps[MAPS_PER_SAMPLE];
+    for (int b = 0; b < MAPS_PER_SAMPLE; ++b)
+        if (!encode_box_map(encoder(), true, sp, base + (b < 3 ? NA_OFF_BUF2 : NA_OFF_BUF3), b % 3, NA_TX, NA_TY, &maps[b]))
             throw LbmError(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-    }
     // small host-to-device copies of values on this stack frame (staged by
     // the driver before the call returns)
     CU(cudaMemcpyAsync(base + NA_OFF_SP, &sp, sizeof(sp), cudaMemcpyHostToDevice, st));
     CU(cudaMemcpyAsync(base + NA_OFF_MAPS, maps, sizeof(maps), cudaMemcpyHostToDevice, st));
+    CU(cudaMemcpyAsync(base + NA_OFF_TILES, tiles.data(), sizeof(Tile) * tiles.size(), cudaMemcpyHostToDevice, st));
     CU(cudaMemcpyAsync(base + NA_OFF_CTYPE, cellType, sizeof(int) * (size_t)Nx * Ny, cudaMemcpyHostToDevice, st));
     k_na_setup<<<64, 256, 0, st>>>(Nx, Ny, pitch, sc.flags, sc.dx, sc.dy, sc.dt, base);
     CU(cudaGetLastError());
@@ -285,15 +289,17 @@ static lbm_status step_noalloc(const lbm_config *cfg, int Nx, int Ny, const int 
     a.fref = reinterpret_cast<const double *>(base + NA_OFF_FREF);
     a.want_residual = 0;
     a.eq_tol = 1e-6;
+    TileRun sweep, general;
+    split_runs(a.tiles, sp.ntile, ns, sweep, general);
     for (int k = 0; k < n_steps; ++k) {
         CU((launch_phase<double, double>(a, 0, sc.rk, a.tiles, sp.ntile, nullptr, 0, st)));
-        k_na_wall<<<64, 256, 0, st>>>(base, NA_OFF_BUF2);
+        if (general.n) k_na_wall<<<64, 256, 0, st>>>(base, NA_OFF_BUF2);
         CU(cudaGetLastError());
-        CU((launch_phase<double, double>(a, 1, sc.rk, a.tiles, sp.ntile, nullptr, 0, st)));
+        stencil_runs<double, double>(a, 1, sc.rk, sweep, general, st);
         if (sc.rk == 1) {
-            k_na_wall<<<64, 256, 0, st>>>(base, NA_OFF_BUF3);
+            if (general.n) k_na_wall<<<64, 256, 0, st>>>(base, NA_OFF_BUF3);
             CU(cudaGetLastError());
-            CU((launch_phase<double, double>(a, 2, 1, a.tiles, sp.ntile, nullptr, 0, st)));
+            stencil_runs<double, double>(a, 2, 1, sweep, general, st);
         }
     }
     k_na_io<<<128, 256, 0, st>>>(Nx, Ny, pitch, d_f, d_h, base, 1);

@@ -381,7 +381,12 @@ class Batch:
         return (int(chosen[0]), int(chosen[1])), {tuple(c): float(t) for c, t in zip(candidates, ms)}
 
     def launches_per_step(self, residual=False):
+        """Kernels of one step taken phase by phase (profile, use_graph=False)."""
         return N.lib().lbm_batch_launches_per_step(self._h, 1 if residual else 0)
+
+    def graph_launches(self, residual=False):
+        """Kernels of one step replayed from a graph."""
+        return N.lib().lbm_batch_graph_launches(self._h, 1 if residual else 0)
 
 
 class Server:
