@@ -3,6 +3,7 @@
 #pragma once
 
 #include "lbm_device.cuh"
+#include "lbm_kernels.h"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -40,24 +41,24 @@ __host__ __device__ constexpr bool box_map_4d(int tx)
     return sizeof(S) == 8 && 2 * box_width<S>(BOX_XY, tx) > 256;
 }
 
-// TMA descriptor of one stage buffer of a sample for one box shape: the 13
-// planes as a 3D tensor (x, y, plane).  The elements are moved as 8-byte
-// words: an FP32 pair, or one value of an FP64 pair (then x counts values).
-// With ghost columns the tensor starts at the left ghosts and spans the pitch
-// (boxes at the x edges then read the images); else it is the domain, and
-// boxes read zeros beyond it.
+// TMA descriptor of one buffer of a sample, its 13 planes as a 3D tensor
+// (x, y, plane), for boxes of bw x bh nodes of one plane.  The elements are
+// moved as 8-byte words: an FP32 pair, or one value of an FP64 pair (then x
+// counts values; four: the pair as a dimension of its own).  With ghost
+// columns the tensor starts at the left ghosts and spans the pitch (boxes at
+// the x edges then read the images); else it is the domain, and boxes read
+// zeros beyond it.
 template <class S>
-bool encode_box_map_t(PFN_cuTensorMapEncodeTiled_v12000 enc, const SampleParams &p, unsigned char *buf, int shape, int tx,
-                      int ty, CUtensorMap *map)
+bool encode_map_t(PFN_cuTensorMapEncodeTiled_v12000 enc, const SampleParams &p, unsigned char *buf, int bw, int bh,
+                  bool four, CUtensorMap *map)
 {
     const cuuint64_t pair = 2 * sizeof(S), nx = (cuuint64_t)(p.gx ? p.pitch : p.nx);
-    const cuuint32_t bw = (cuuint32_t)box_width<S>(shape, tx), bh = (cuuint32_t)box_height(shape, ty);
     unsigned char *base = buf + (size_t)(p.state_off - 2 * p.gx) * sizeof(S);
     const cuuint32_t estr[4] = {1, 1, 1, 1};
-    if (box_map_4d<S>(tx)) {
+    if (four) {
         const cuuint64_t dims[4] = {2, nx, (cuuint64_t)p.ny, (cuuint64_t)NQ};
         const cuuint64_t strides[3] = {pair, p.pitch * pair, (cuuint64_t)p.plane * pair};
-        const cuuint32_t box[4] = {2, bw, bh, 1};
+        const cuuint32_t box[4] = {2, (cuuint32_t)bw, (cuuint32_t)bh, 1};
         return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -65,17 +66,29 @@ bool encode_box_map_t(PFN_cuTensorMapEncodeTiled_v12000 enc, const SampleParams 
     const cuuint32_t w = (cuuint32_t)(pair / 8);
     const cuuint64_t dims[3] = {nx * w, (cuuint64_t)p.ny, (cuuint64_t)NQ};
     const cuuint64_t strides[2] = {p.pitch * pair, (cuuint64_t)p.plane * pair};
-    const cuuint32_t box[3] = {bw * w, bh, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)bw * w, (cuuint32_t)bh, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-inline bool encode_box_map(PFN_cuTensorMapEncodeTiled_v12000 enc, bool f64, const SampleParams &p, unsigned char *buf,
-                           int shape, int tx, int ty, CUtensorMap *map)
+// The MAPS_PER_SAMPLE descriptors of a sample.
+template <class S>
+bool encode_box_maps_t(PFN_cuTensorMapEncodeTiled_v12000 enc, const SampleParams &p, unsigned char *buf2,
+                       unsigned char *buf3, int tx, int ty, CUtensorMap *maps)
 {
-    return f64 ? encode_box_map_t<double>(enc, p, buf, shape, tx, ty, map)
-               : encode_box_map_t<float>(enc, p, buf, shape, tx, ty, map);
+    for (int b = 0; b < 6; ++b)
+        if (!encode_map_t<S>(enc, p, b < 3 ? buf2 : buf3, box_width<S>(b % 3, tx), box_height(b % 3, ty),
+                             box_map_4d<S>(tx), &maps[b]))
+            return false;
+    return true;
+}
+
+inline bool encode_box_maps(PFN_cuTensorMapEncodeTiled_v12000 enc, bool f64, const SampleParams &p, unsigned char *buf2,
+                            unsigned char *buf3, int tx, int ty, CUtensorMap *maps)
+{
+    return f64 ? encode_box_maps_t<double>(enc, p, buf2, buf3, tx, ty, maps)
+               : encode_box_maps_t<float>(enc, p, buf2, buf3, tx, ty, maps);
 }
 
 }  // namespace uqlbm

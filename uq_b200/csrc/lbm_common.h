@@ -95,8 +95,7 @@ void cut_tiles(const uint8_t *flags, const SampleParams &p, int tx, int ty, int 
 // cut_tiles made them
 void needed_walls(const SampleParams &p, int tx, int ty, const Tile *tiles, const std::vector<WallNode> &walls,
                   std::vector<WallNode> &out);
-// TMA descriptors of one sample (MAPS_PER_SAMPLE of them): stage buffers 2
-// and 3, each with the stencil kernels' three box shapes
+// TMA descriptors of one sample (MAPS_PER_SAMPLE of them)
 void encode_stage_maps(int prec, const SampleParams &p, unsigned char *buf2, unsigned char *buf3, int tx, int ty,
                        CUtensorMap *maps);
 void check_tile_shape(int x, int y);

@@ -73,12 +73,15 @@ struct SampleParams {
 constexpr int GHOST_X = 4;       // = the staged box's x halo
 constexpr int GHOST_SLACK = 32;  // state elements before plane 0 of a sample with ghosts (keeps it aligned)
 
+// What a block needs before it can ask for its boxes and sweep them (the
+// sample's parameters arrive meanwhile).
 struct Tile {
     int sample;
     int x0, y0;
-    int gid;   // index of the tile in the batch's full tile list
-    int kind;  // TILE_* bits
-    int pad[3];
+    int gid;      // index of the tile in the batch's full tile list
+    int kind;     // TILE_* bits
+    float c;      // (float)SampleParams::c
+    double eps1;  // SampleParams::eps1
 };
 
 // Kinds of tiles in the stencil phases.  A sweep tile's fluxes all come from
@@ -697,16 +700,21 @@ struct FaceArg<double> {
     double2 eps;
 };
 template <class C>
-__device__ __forceinline__ FaceArg<C> face_arg(const SampleParams &sp, int comp)
+__device__ __forceinline__ FaceArg<C> face_arg(float c, double eps1, int comp)
 {
     const bool two = comp == 2 || comp == -2;
     if constexpr (sizeof(C) == 4) {
-        const float c = (float)sp.c, ae = two ? 2.f * c : c;
+        const float ae = two ? 2.f * c : c;
         return FaceArg<C>{make_float2(ae, ae), make_float2(0.5f * ae, 0.5f * ae)};
     } else {
-        const double e = two ? 0.25 * sp.eps1 : sp.eps1;
+        const double e = two ? 0.25 * eps1 : eps1;
         return FaceArg<C>{make_double2(e, e)};
     }
+}
+template <class C>
+__device__ __forceinline__ FaceArg<C> face_arg(const SampleParams &sp, int comp)
+{
+    return face_arg<C>((float)sp.c, sp.eps1, comp);
 }
 
 // minmod with the reference's case order (cpuLBM.cpp:1130-1145): same
@@ -750,18 +758,11 @@ __device__ __forceinline__ double2 face_div(double2 n, double2 d)
 
 // ---- FP32.  w = |e| s / 2: half the scaled value, so that the smoothness
 // terms need no factors (a quarter of a slope's square is the square of its
-// half; powers of two round nothing).
-struct WenoPoint32 {
-    float2 w, q;  // |e| s / 2, |e| s
-};
+// half).  Factors of two round nothing, so they are moved to where they cost
+// no operation.
 struct WenoCurv32 {
     float2 d, k;  // half the second difference, 13/3 of it
 };
-__device__ __forceinline__ WenoPoint32 weno_point(float2 s, const FaceArg<float> &g)
-{
-    const float2 w = xmul(g.aeh, s);
-    return WenoPoint32{w, xadd(w, w)};
-}
 __device__ __forceinline__ WenoCurv32 weno_curv(float2 w0, float2 w1, float2 w2)
 {
     const float2 d = xfma(kc<float2>(-2), w1, xadd(w0, w2));
@@ -769,37 +770,37 @@ __device__ __forceinline__ WenoCurv32 weno_curv(float2 w0, float2 w1, float2 w2)
 }
 // the face from its five points and the curvatures at the middle three
 template <bool WIDE>
-__device__ __forceinline__ float2 weno_face(const WenoPoint32 &p0, const WenoPoint32 &p1, const WenoPoint32 &p2,
-                                            const WenoPoint32 &p3, const WenoPoint32 &p4, const WenoCurv32 &c0,
+__device__ __forceinline__ float2 weno_face(float2 p0, float2 p1, float2 p2, float2 p3, float2 p4, const WenoCurv32 &c0,
                                             const WenoCurv32 &c1, const WenoCurv32 &c2)
 {
     using V = float2;
     // half the one-sided slopes of the three stencils
-    const V l0 = xfma(kc<V>(3), p2.w, xfma(kc<V>(-4), p1.w, p0.w));
-    const V l1 = xsub(p1.w, p3.w);
-    const V l2 = xfma(kc<V>(-4), p3.w, xfma(kc<V>(3), p2.w, p4.w));
+    const V l0 = xfma(kc<V>(3), p2, xfma(kc<V>(-4), p1, p0));
+    const V l1 = xsub(p1, p3);
+    const V l2 = xfma(kc<V>(-4), p3, xfma(kc<V>(3), p2, p4));
     // eps + b_k
     const V a0 = xfma(c0.k, c0.d, xfma(l0, l0, kc<V>(1e-6)));
     const V a1 = xfma(c1.k, c1.d, xfma(l1, l1, kc<V>(1e-6)));
     const V a2 = xfma(c2.k, c2.d, xfma(l2, l2, kc<V>(1e-6)));
-    V w0, w1, w2;  // weights, the middle one negative (its candidate is too)
+    V w0, w1, w2;  // weights; of the middle one minus a half
+    constexpr float k1 = -0.5f * (float)0.6;
     if constexpr (WIDE) {
         const V m = xmin(a0, xmin(a1, a2));
         const V s0 = face_div(m, a0), s1 = face_div(m, a1), s2 = face_div(m, a2);
         w0 = xmul(kc<V>(0.1), xmul(s0, s0));
-        w1 = xmul(kc<V>(-0.6), xmul(s1, s1));
+        w1 = xmul(make_float2(k1, k1), xmul(s1, s1));
         w2 = xmul(kc<V>(0.3), xmul(s2, s2));
     } else {
         const V b0 = xmul(a0, a0), b1 = xmul(a1, a1), b2 = xmul(a2, a2);
         w0 = xmul(kc<V>(0.1), xmul(b1, b2));
-        w1 = xmul(kc<V>(-0.6), xmul(b0, b2));
+        w1 = xmul(make_float2(k1, k1), xmul(b0, b2));
         w2 = xmul(kc<V>(0.3), xmul(b0, b1));
     }
-    // candidate reconstructions (times 3)
-    const V r0 = xfma(kc<V>(11), p2.w, xfma(kc<V>(-7), p1.w, p0.q));
-    const V r1 = xfma(kc<V>(-2), p3.w, xfma(kc<V>(-5), p2.w, p1.w));
-    const V r2 = xsub(xfma(kc<V>(5), p3.w, p2.q), p4.w);
-    return face_div(xfma(w2, r2, xfma(w1, r1, xmul(w0, r0))), xmul(kc<V>(3), xadd(xsub(w0, w1), w2)));
+    // candidate reconstructions, times 3/2 (the middle one: times -3)
+    const V r0 = xfma(kc<V>(5.5), p2, xfma(kc<V>(-3.5), p1, p0));
+    const V r1 = xfma(kc<V>(-2), p3, xfma(kc<V>(-5), p2, p1));
+    const V r2 = xfma(kc<V>(-0.5), p4, xfma(kc<V>(2.5), p3, p2));
+    return face_div(xfma(w2, r2, xfma(w1, r1, xmul(w0, r0))), xmul(kc<V>(1.5), xadd(xfma(kc<V>(-2), w1, w0), w2)));
 }
 // NND (cpuLBM.cpp:1328-1356): c = |e| s1, the differences to |e| s2, |e| s0
 __device__ __forceinline__ float2 nnd_face(float2 s0, float2 s1, float2 s2, float2 c, const FaceArg<float> &g)
@@ -847,10 +848,10 @@ __device__ __forceinline__ float2 face5(float2 s0, float2 s1, float2 s2, float2 
 {
     if constexpr (FM == 0) return nnd_face(s1, s2, s3, xmul(g.ae, s2), g);
     else {
-        const WenoPoint32 p0 = weno_point(s0, g), p1 = weno_point(s1, g), p2 = weno_point(s2, g), p3 = weno_point(s3, g),
-                          p4 = weno_point(s4, g);
-        return weno_face<FM == 2>(p0, p1, p2, p3, p4, weno_curv(p0.w, p1.w, p2.w), weno_curv(p1.w, p2.w, p3.w),
-                                  weno_curv(p2.w, p3.w, p4.w));
+        const float2 p0 = xmul(g.aeh, s0), p1 = xmul(g.aeh, s1), p2 = xmul(g.aeh, s2), p3 = xmul(g.aeh, s3),
+                     p4 = xmul(g.aeh, s4);
+        return weno_face<FM == 2>(p0, p1, p2, p3, p4, weno_curv(p0, p1, p2), weno_curv(p1, p2, p3),
+                                  weno_curv(p2, p3, p4));
     }
 }
 template <int FM>
@@ -894,13 +895,12 @@ __device__ __forceinline__ void line_diffs(const float2 (&v)[LEN + 5], const Fac
             prev = F;
         }
     } else {
-        WenoPoint32 p0 = weno_point(v[0], g), p1 = weno_point(v[1], g), p2 = weno_point(v[2], g),
-                    p3 = weno_point(v[3], g);
-        WenoCurv32 c0 = weno_curv(p0.w, p1.w, p2.w), c1 = weno_curv(p1.w, p2.w, p3.w);
+        float2 p0 = xmul(g.aeh, v[0]), p1 = xmul(g.aeh, v[1]), p2 = xmul(g.aeh, v[2]), p3 = xmul(g.aeh, v[3]);
+        WenoCurv32 c0 = weno_curv(p0, p1, p2), c1 = weno_curv(p1, p2, p3);
 #pragma unroll
         for (int n = -1; n < LEN; ++n) {
-            const WenoPoint32 p4 = weno_point(v[n + 5], g);
-            const WenoCurv32 c2 = weno_curv(p2.w, p3.w, p4.w);
+            const float2 p4 = xmul(g.aeh, v[n + 5]);
+            const WenoCurv32 c2 = weno_curv(p2, p3, p4);
             const float2 F = hook(n, weno_face<FM == 2>(p0, p1, p2, p3, p4, c0, c1, c2));
             if (n >= 0) out[n] = xsub(F, prev);
             prev = F;

@@ -353,7 +353,7 @@ void cut_tiles(const uint8_t *flags, const SampleParams &p, int tx, int ty, int 
     }
     for (int y0 = 0; y0 < ny; y0 += ty)
         for (int x0 = 0; x0 < nx; x0 += tx) {
-            Tile t{sample, x0, y0, (int)out.size(), base, {0, 0, 0}};
+            Tile t{sample, x0, y0, (int)out.size(), base, (float)p.c, p.eps1};
             const int xe = std::min(x0 + tx, nx), ye = std::min(y0 + ty, ny);  // the tile's nodes
             const bool w = x0 < 3, e = x0 + tx + 3 > nx, s = y0 < 3, n = y0 + ty + 3 > ny;
             bool fixed = false;  // permanent nodes in the tile, or solids in sight
@@ -415,15 +415,12 @@ void needed_walls(const SampleParams &p, int tx, int ty, const Tile *tiles, cons
             out.push_back(w);
 }
 
-// TMA descriptors of a sample: stage buffers 2 and 3 over the 13 planes of
-// pairs, each with the stencil kernels' three box shapes (encode_box_map).
+// TMA descriptors of a sample (see encode_box_maps).
 void encode_stage_maps(int prec, const SampleParams &p, unsigned char *buf2, unsigned char *buf3, int tx, int ty,
                        CUtensorMap *maps)
 {
-    auto enc = tensor_map_encoder();
-    for (int b = 0; b < MAPS_PER_SAMPLE; ++b)
-        if (!encode_box_map(enc, prec == LBM_PREC_F64, p, b < 3 ? buf2 : buf3, b % 3, tx, ty, &maps[b]))
-            throw LbmError(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    if (!encode_box_maps(tensor_map_encoder(), prec == LBM_PREC_F64, p, buf2, buf3, tx, ty, maps))
+        throw LbmError(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
 }
 
 }  // namespace uqlbm

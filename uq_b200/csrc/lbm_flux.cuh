@@ -23,6 +23,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 namespace uqlbm {
 
 // pairs of a box, padded to 128 bytes
@@ -47,15 +49,15 @@ __host__ __device__ constexpr int part_index(int i, int axis)
 
 // Shared memory.  Default tile: the 12 boxes, whose space takes the parts of
 // the direction once read, and the x parts of the diagonals apart (their
-// boxes are still being swept along y).  Other tile shapes: `slots` boxes at
-// a time and all 16 parts apart.  General tiles: the parts only.
+// boxes are still being swept along y).  Other tile shapes: `slots` boxes at a time
+// and all 16 parts apart.  General tiles: the parts only.
 struct FluxSmem {
-    int slots;        // boxes resident at a time
-    int slot_pairs;   // pairs per slot (not the default tile)
-    int part_off;     // the parts (default tile: the diagonals' x parts), in pairs
-    int wall_off;     // saved wall faces, in pairs
-    int bar_off;      // mbarriers, in pairs
-    size_t bytes;     // with 128 bytes of base-alignment slack
+    int slots;       // boxes resident at a time
+    int slot_pairs;  // pairs per slot (not the default tile)
+    int part_off;    // the parts (default tile: the diagonals' x parts), in pairs
+    int wall_off;    // saved wall faces, in pairs
+    int bar_off;     // mbarriers, in pairs
+    size_t bytes;    // with 128 bytes of base-alignment slack
 };
 
 // default tile: pairs before direction i's box
@@ -156,10 +158,10 @@ __device__ __forceinline__ void issue_box(Pair<S> *dst, const CUtensorMap *maps,
 // puts there.  (The wall row's own nodes are solid: their x lines are not
 // used.)
 template <class S>
-__device__ __noinline__ void fix_box(Pair<S> *box, const SampleParams *gsp, const StageView<S> v, const Tile t, int tx,
-                                     int ty, int i, int id, int n)
+__device__ __noinline__ void fix_box(Pair<S> *box, const SampleParams &sp, const S *stage, const Tile t, int tx, int ty,
+                                     int i, int id, int n)
 {
-    const SampleParams &sp = *gsp;
+    const StageView<S> v{stage + sp.state_off, nullptr, (int)sp.plane, sp.pitch};
     const int sh = box_shape(i);
     const BoxPlace g = box_place<S>(sh, tx);
     const int bx0 = t.x0 - g.cx, by0 = t.y0 - g.ry;  // domain place of the box's first cell
@@ -167,30 +169,28 @@ __device__ __noinline__ void fix_box(Pair<S> *box, const SampleParams *gsp, cons
     const bool ws = (t.kind & TILE_WALLS) != 0, wn = (t.kind & TILE_WALLN) != 0;
     auto cell = [&](int x, int y) -> Pair<S> & { return box[(y - by0) * g.rs + (x - bx0)]; };
     if (sh != BOX_Y && !(px && sp.gx)) {
-        const int w = 2 * HALO + tx;  // columns x0 - 3 .. x0 + tx + 2
-        for (int e = id; e < w * ty; e += n) {
-            const int r = e / w, x = t.x0 - HALO + (e - r * w), y = t.y0 + r;
-            if (x >= 0 && x < sp.nx) continue;
+        // the columns left of 0 and from nx on that a node of the tile sees
+        const int left = max(HALO - t.x0, 0), right = min(max(t.x0 + tx + HALO - sp.nx, 0), HALO);
+        for (int e = id; e < (left + right) * ty; e += n) {
+            const int c = e / ty, y = t.y0 + (e - c * ty), x = c < left ? t.x0 - HALO + c : sp.nx + (c - left);
             if (y >= sp.ny - (wn ? 1 : 0) || (ws && y < 1)) continue;  // no line that is used
-            if (px) {
-                cell(x, y) = ldv(v, i, ((x % sp.nx) + sp.nx) % sp.nx, y);
-            } else if (x < 0 || x < sp.nx + HALO) {
-                cell(x, y) = cell(x < 0 ? 0 : sp.nx - 1, y);
-            }
+            cell(x, y) = px ? ldv(v, i, ((x % sp.nx) + sp.nx) % sp.nx, y) : cell(x < 0 ? 0 : sp.nx - 1, y);
         }
     }
     if (sh != BOX_X) {
-        const int h = 2 * HALO + ty;
-        for (int e = id; e < h * tx; e += n) {
-            const int r = e / tx, x = t.x0 + (e - r * tx), y = t.y0 - HALO + r;
-            if (x >= sp.nx || (y >= (ws ? 1 : 0) && y < (wn ? sp.ny - 1 : sp.ny))) continue;
-            if (py) {
-                cell(x, y) = ldv(v, i, x, ((y % sp.ny) + sp.ny) % sp.ny);
-            } else if (y < 1) {
-                cell(x, y) = ws ? extrapolate(cell(x, 1), cell(x, 2)) : cell(x, 0);
-            } else if (y < sp.ny + HALO) {
-                cell(x, y) = wn ? extrapolate(cell(x, sp.ny - 2), cell(x, sp.ny - 3)) : cell(x, sp.ny - 1);
-            }
+        // the rows before `first` and from `last` on that a node of the tile
+        // sees; a wall row counts as outside
+        const int first = min(t.y0 + ty + HALO, ws ? 1 : 0), last = max(t.y0 - HALO, wn ? sp.ny - 1 : sp.ny);
+        const int end = min(t.y0 + ty, sp.ny) + HALO;
+        for (int col = id; col < tx; col += n) {
+            const int x = t.x0 + col;
+            if (x >= sp.nx) continue;
+            for (int y = t.y0 - HALO; y < first; ++y)
+                cell(x, y) = py ? ldv(v, i, x, ((y % sp.ny) + sp.ny) % sp.ny)
+                           : ws ? extrapolate(cell(x, 1), cell(x, 2)) : cell(x, 0);
+            for (int y = last; y < end; ++y)
+                cell(x, y) = py ? ldv(v, i, x, ((y % sp.ny) + sp.ny) % sp.ny)
+                           : wn ? extrapolate(cell(x, sp.ny - 2), cell(x, sp.ny - 3)) : cell(x, sp.ny - 1);
         }
     }
 }
@@ -266,9 +266,22 @@ __device__ __forceinline__ void sweep_x(const Pair<S> *box, BoxPlace g, bool pos
         line_diffs<FM, LEN>(v, fa, out, NoHook());
     }
 }
-// node n of a line lies at column (row) c0 + n, or counted back
+// node n of a line lies at column (row) n of its segment, or counted back;
+// both written out, so that every address is a constant distance from one
 template <class V, int LEN>
-__device__ __forceinline__ void store_line(V *part, const V (&out)[LEN], bool pos, int step, int lim)
+__device__ __forceinline__ void store_line(V *part, const V (&out)[LEN], bool pos, int step)
+{
+    if (pos) {
+#pragma unroll
+        for (int n = 0; n < LEN; ++n) part[n * step] = out[n];
+    } else {
+#pragma unroll
+        for (int n = 0; n < LEN; ++n) part[(LEN - 1 - n) * step] = out[n];
+    }
+}
+// the same of a line that may reach beyond the tile (other tile shapes)
+template <class V, int LEN>
+__device__ __forceinline__ void store_line_to(V *part, const V (&out)[LEN], bool pos, int step, int lim)
 {
 #pragma unroll
     for (int n = 0; n < LEN; ++n) {
@@ -277,22 +290,28 @@ __device__ __forceinline__ void store_line(V *part, const V (&out)[LEN], bool po
     }
 }
 
-template <class S, int FM, int LEN, bool HOOK>
-__device__ __forceinline__ void sweep_y(const Pair<S> *box, BoxPlace g, bool pos, int col, int r0, int last, const FaceArg<S> &fa,
-                                        Pair<S> (&out)[LEN], const WallHook<S> &hook)
+// the same along y, column `col`, rows r0 .. r0 + LEN - 1.  last: the last row
+// of the box, where a line may reach beyond it (LAST, other tile shapes)
+template <class S, int FM, int LEN, bool HOOK, bool LAST>
+__device__ __forceinline__ void sweep_y(const Pair<S> *box, BoxPlace g, bool pos, int col, int r0, int last,
+                                        const FaceArg<S> &fa, Pair<S> (&out)[LEN], const WallHook<S> &hook)
 {
     using V = Pair<S>;
     V v[LEN + 5];
     const V *p = box + col + g.cx;
-    const int s = pos ? 1 : -1, r = r0 + HALO + (pos ? -3 : LEN + 2);
-    if (last < 0) {  // every row of the line is in the box
-        const V *q = p + r * g.rs;
-        const int st = s * g.rs;
-#pragma unroll
-        for (int k = 0; k < LEN + 5; ++k) v[k] = q[st * k];
-    } else {
+    if constexpr (LAST) {
+        const int s = pos ? 1 : -1, r = r0 + HALO + (pos ? -3 : LEN + 2);
 #pragma unroll
         for (int k = 0; k < LEN + 5; ++k) v[k] = p[min(r + s * k, last) * g.rs];
+    } else {
+        const V *q = p + r0 * g.rs;
+        if (pos) {
+#pragma unroll
+            for (int k = 0; k < LEN + 5; ++k) v[k] = q[k * g.rs];
+        } else {
+#pragma unroll
+            for (int k = 0; k < LEN + 5; ++k) v[k] = q[(LEN + 5 - k) * g.rs];
+        }
     }
     if constexpr (HOOK) line_diffs<FM, LEN>(v, fa, out, hook);
     else line_diffs<FM, LEN>(v, fa, out, NoHook());
@@ -301,12 +320,12 @@ __device__ __forceinline__ void sweep_y(const Pair<S> *box, BoxPlace g, bool pos
 // one warp of a default tile: direction ix along x, then iy along y
 // (equal for the diagonals)
 template <class S, int FM>
-__device__ __forceinline__ bool sweep_warp(const Tile &t, const SampleParams *gsp, const StageView<S> v, Pair<S> *sm,
-                                           uint64_t *bars, int warp, int lane)
+__device__ __forceinline__ bool sweep_warp(const Tile &t, const SampleParams &sp, const S *stage, Pair<S> *sm, S *save,
+                                           uint64_t *bars, uint32_t parity, int warp, int lane)
 {
     using V = Pair<S>;
     constexpr FluxSmem L = flux_smem<S>(TILE_CX, TILE_CY, true, true, 12);
-    constexpr int PR = TILE_CX + 1;
+    constexpr int PR = TILE_CX + 1, PP = part_pairs(TILE_CX, TILE_CY);
     const bool diag = warp >= 4;
     const int ix = diag ? warp + 1 : warp < 2 ? 1 + 2 * warp : 5 + 2 * warp;
     const int iy = diag ? warp + 1 : ix + 1;
@@ -316,41 +335,40 @@ __device__ __forceinline__ bool sweep_warp(const Tile &t, const SampleParams *gs
         V *box = sm + box_start<S>(ix);
         const BoxPlace g = diag ? box_place<S>(BOX_XY, TILE_CX) : box_place<S>(BOX_X, TILE_CX);
         const bool pos = lat_ex(ix) > 0;
-        const FaceArg<S> fa = face_arg<S>(*gsp, lat_ex(ix));
-        ok = mbar_wait_bounded(&bars[ix - 1], 0, TMA_WAIT_POLLS);
+        const FaceArg<S> fa = face_arg<S>(t.c, t.eps1, lat_ex(ix));
+        ok = mbar_wait_bounded(&bars[ix - 1], parity, TMA_WAIT_POLLS);
         if (fix) {
-            fix_box<S>(box, gsp, v, t, TILE_CX, TILE_CY, ix, lane, 32);
+            fix_box<S>(box, sp, stage, t, TILE_CX, TILE_CY, ix, lane, 32);
             __syncwarp();
         }
         const int row = lane & 7, c0 = (lane >> 3) * 8;
         V out[8];
         sweep_x<S, FM, 8>(box, g, pos, row, c0, fa, out);
-        V *part = diag ? sm + L.part_off + (ix - 5) * part_pairs(TILE_CX, TILE_CY) : box;
+        V *part = diag ? sm + L.part_off + (ix - 5) * PP : box;
         if (!diag) __syncwarp();
-        store_line<V, 8>(part + row * PR + c0, out, pos, 1, 8);
+        store_line<V, 8>(part + row * PR + c0, out, pos, 1);
     }
     {
         V *box = sm + box_start<S>(iy);
-        const BoxPlace g = diag ? box_place<S>(BOX_XY, TILE_CX) : box_place<S>(BOX_Y, TILE_CX);
         const bool pos = lat_ey(iy) > 0;
-        const FaceArg<S> fa = face_arg<S>(*gsp, lat_ey(iy));
+        const FaceArg<S> fa = face_arg<S>(t.c, t.eps1, lat_ey(iy));
         V out[8];
         if (!diag) {
-            ok = mbar_wait_bounded(&bars[iy - 1], 0, TMA_WAIT_POLLS) && ok;
+            ok = mbar_wait_bounded(&bars[iy - 1], parity, TMA_WAIT_POLLS) && ok;
             if (fix) {
-                fix_box<S>(box, gsp, v, t, TILE_CX, TILE_CY, iy, lane, 32);
+                fix_box<S>(box, sp, stage, t, TILE_CX, TILE_CY, iy, lane, 32);
                 __syncwarp();
             }
         }
-        if (t.kind & (TILE_WALLS | TILE_WALLN)) {
-            const WallHook<S> hook{pos ? t.y0 : t.y0 + 7, pos ? 1 : -1, gsp->ny, t.kind, lane, TILE_CX, wall_slot_in(iy),
-                                   reinterpret_cast<S *>(sm + L.wall_off)};
-            sweep_y<S, FM, 8, true>(box, g, pos, lane, 0, -1, fa, out, hook);
-        } else {
-            sweep_y<S, FM, 8, false>(box, g, pos, lane, 0, -1, fa, out, WallHook<S>{});
-        }
+        const bool walls = (t.kind & (TILE_WALLS | TILE_WALLN)) != 0;
+        const WallHook<S> hook{pos ? t.y0 : t.y0 + 7, pos ? 1 : -1, walls ? sp.ny : 0, t.kind, lane, TILE_CX,
+                               wall_slot_in(iy), save};
+        // (one copy of the sweep for both box widths)
+        const BoxPlace g = diag ? box_place<S>(BOX_XY, TILE_CX) : box_place<S>(BOX_Y, TILE_CX);
+        if (walls) sweep_y<S, FM, 8, true, false>(box, g, pos, lane, 0, 0, fa, out, hook);
+        else sweep_y<S, FM, 8, false, false>(box, g, pos, lane, 0, 0, fa, out, hook);
         __syncwarp();
-        store_line<V, 8>(box + lane, out, pos, PR, 8);
+        store_line<V, 8>(box + lane, out, pos, PR);
     }
     return ok;
 }
@@ -358,7 +376,7 @@ __device__ __forceinline__ bool sweep_warp(const Tile &t, const SampleParams *gs
 // other tile shapes: the boxes resident, in lines of 4 nodes spread over the
 // block's threads
 template <class S, int FM>
-__device__ void sweep_block(const Tile &t, const SampleParams *gsp, const Pair<S> *slots, int slot_pairs, Pair<S> *parts,
+__device__ void sweep_block(const Tile &t, const SampleParams &sp, const Pair<S> *slots, int slot_pairs, Pair<S> *parts,
                             S *save, int tx, int ty, int i0, int ndir, int tid, int nt)
 {
     using V = Pair<S>;
@@ -374,17 +392,17 @@ __device__ void sweep_block(const Tile &t, const SampleParams *gsp, const Pair<S
             if (sh == BOX_Y) continue;
             const int seg = q / ty, row = q - seg * ty;
             const bool pos = lat_ex(i) > 0;
-            sweep_x<S, FM, 4>(box, g, pos, row, 4 * seg, face_arg<S>(*gsp, lat_ex(i)), out);
-            store_line<V, 4>(parts + part_index(i, 0) * PP + row * PR + 4 * seg, out, pos, 1, 4);
+            sweep_x<S, FM, 4>(box, g, pos, row, 4 * seg, face_arg<S>(t.c, t.eps1, lat_ex(i)), out);
+            store_line_to<V, 4>(parts + part_index(i, 0) * PP + row * PR + 4 * seg, out, pos, 1, 4);
         } else {
             if (sh == BOX_X) continue;
             const int p = q - nxi, seg = p / tx, col = p - seg * tx;
             const bool pos = lat_ey(i) > 0;
-            const WallHook<S> hook{pos ? t.y0 + 4 * seg : t.y0 + 4 * seg + 3, pos ? 1 : -1, gsp->ny, t.kind, col, tx,
+            const WallHook<S> hook{pos ? t.y0 + 4 * seg : t.y0 + 4 * seg + 3, pos ? 1 : -1, sp.ny, t.kind, col, tx,
                                    wall_slot_in(i), save};
-            sweep_y<S, FM, 4, true>(box, g, pos, col, 4 * seg, box_height(sh, ty) - 1, face_arg<S>(*gsp, lat_ey(i)), out,
+            sweep_y<S, FM, 4, true, true>(box, g, pos, col, 4 * seg, box_height(sh, ty) - 1, face_arg<S>(t.c, t.eps1, lat_ey(i)), out,
                                     hook);
-            store_line<V, 4>(parts + part_index(i, 1) * PP + 4 * seg * PR + col, out, pos, PR, ty - 4 * seg);
+            store_line_to<V, 4>(parts + part_index(i, 1) * PP + 4 * seg * PR + col, out, pos, PR, ty - 4 * seg);
         }
     }
 }
@@ -402,196 +420,131 @@ __device__ __noinline__ Pair<S> node_face(const SampleParams &sp, const StageVie
     return flux_axis<S, S>(sp, v, x, y, i, axis, fl);
 }
 
+// the whole block of a default tile: each warp its directions
 template <class S>
-struct FluxBlocks {
-    static constexpr int value = 2;
-};
-template <int MODE>
-struct SweepBlocksF32 {
-    static constexpr int value = MODE == 2 ? 3 : 2;
+__device__ __forceinline__ bool sweep_tile(const Tile &t, const SampleParams &sp, const S *stage, Pair<S> *sm, S *save,
+                                           uint64_t *bars, uint32_t parity, int warp, int lane)
+{
+    const int fm = tile_fm(t.kind);
+    // FP64 has one form of the weights
+    if (sizeof(S) == 8 ? fm != 0 : fm == 1) return sweep_warp<S, 1>(t, sp, stage, sm, save, bars, parity, warp, lane);
+    if (fm == 2) return sweep_warp<S, sizeof(S) == 4 ? 2 : 1>(t, sp, stage, sm, save, bars, parity, warp, lane);
+    return sweep_warp<S, 0>(t, sp, stage, sm, save, bars, parity, warp, lane);
+}
+
+// a warp's lane 0 asks for the boxes of the warp's directions (maps: the stage
+// buffer's three)
+template <class S>
+__device__ __forceinline__ void issue_warp(const Tile &t, const CUtensorMap *maps, Pair<S> *sm, uint64_t *bars, int warp)
+{
+    const bool diag = warp >= 4;
+    const int ix = diag ? warp + 1 : warp < 2 ? 1 + 2 * warp : 5 + 2 * warp;
+    const int gx = (t.kind & TILE_GHOST) ? GHOST_X : 0;
+    issue_box<S>(sm + box_start<S>(ix), maps, t.x0, t.y0, gx, TILE_CX, TILE_CY, ix, &bars[ix - 1]);
+    if (!diag) issue_box<S>(sm + box_start<S>(ix + 1), maps, t.x0, t.y0, gx, TILE_CX, TILE_CY, ix + 1, &bars[ix]);
+}
+
+// a node's flux differences in shared memory.  OVER: the default tile's, over
+// the boxes (sm: the tile's copy); else in the 16 part arrays (sm: the first)
+template <class S, bool OVER>
+struct NodeParts {
+    Pair<S> *sm;
+    int pn, PP;  // the node's place in an array; pairs per array
+    __device__ __forceinline__ Pair<S> &operator()(int i, int axis) const
+    {
+        if constexpr (OVER) {
+            constexpr FluxSmem L = flux_smem<S>(TILE_CX, TILE_CY, true, true, 12);
+            if (box_shape(i) == BOX_XY && axis == 0)
+                return sm[L.part_off + (i - 5) * part_pairs(TILE_CX, TILE_CY) + pn];
+            return sm[box_start<S>(i) + pn];
+        } else {
+            return sm[part_index(i, axis) * PP + pn];
+        }
+    }
 };
 
-// MODE: 1 = RK3 stage 3 (fluxes of buffer 2), 2 = RK3 final (buffer 3),
-// 3 = RK1 update, 4 = EULER update, 5 = EULER_EQ update (buffer 2)
-// PATH: FLUX_SWEEP or FLUX_GENERAL, the tiles of one kind per launch (a
-// block given the other kind returns at once).
-// TC: the default tile shape, compiled in; other shapes are read from the
-// arguments and give every node the same bits.
-template <class S, int MODE, int PATH, bool TC>
-__global__ void __launch_bounds__(256, (sizeof(S) == 4 && PATH == FLUX_SWEEP && TC) ? SweepBlocksF32<MODE>::value : 2)
-k_flux(KArgs<S> a)
+// whether the per-node half loads the state before the block's barrier
+template <class S>
+__host__ __device__ constexpr bool flux_early(int mode)
+{
+    return sizeof(S) == 8 || mode == 3;
+}
+
+// The per-node half of a stencil phase (MODE as k_flux): the node's
+// divergences from its parts, then the RK3 stage 3 or the update.  The
+// block's barrier between the sweeps and this lies inside, after the loads
+// that do not depend on the sweeps.
+template <class S, int MODE, bool SWEEP, class PART>
+__device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, const SampleParams &sp, const PART &part,
+                                           const S *save, double *red, int TX, int NT, int tid)
 {
     using C = S;
     using V = Pair<S>;
-    extern __shared__ __align__(128) unsigned char smem_dyn[];
-    __shared__ double red[32];
-    __shared__ SampleParams s_sp;  // kept out of registers: read as needed
-    constexpr bool SWEEP = PATH == FLUX_SWEEP;
-    const int TX = TC ? TILE_CX : a.tx, TY = TC ? TILE_CY : a.ty, NT = TX * TY;
-    const int tid = threadIdx.x;
-    V *sm = reinterpret_cast<V *>(smem_dyn + ((128 - (smem_u32(smem_dyn) & 127)) & 127));
-    const Tile t = a.tiles[blockIdx.x];
-    if (tile_sweep(t) != SWEEP) return;
-    constexpr int PH = MODE == 2 ? 2 : 1;
-    const SampleParams *gsp = a.samples + t.sample;
-    const CUtensorMap *maps = a.tmaps + MAPS_PER_SAMPLE * t.sample + (PH == 1 ? 0 : 3);
-    const S *stage = PH == 1 ? a.buf2 : a.buf3;
-    const int PR = TX + 1, PP = part_pairs(TX, TY);
-    constexpr FluxSmem LC = flux_smem<S>(TILE_CX, TILE_CY, true, true, 12);
-    FluxSmem Lr{};
-    if constexpr (!TC) Lr = flux_smem<S>(TX, TY, false, SWEEP, SWEEP ? a.slots : 0);
-    const int part_off = TC ? (SWEEP ? LC.part_off : 0) : Lr.part_off;
-    const int wall_off = TC ? LC.wall_off : Lr.wall_off;
-
-    for (int k = tid; k < (int)(sizeof(SampleParams) / 4); k += NT)
-        reinterpret_cast<int *>(&s_sp)[k] = reinterpret_cast<const int *>(gsp)[k];
-    if constexpr (SWEEP) {
-        uint64_t *bars = reinterpret_cast<uint64_t *>(sm + (TC ? LC.bar_off : Lr.bar_off));
-        const int fm = tile_fm(t.kind);
-        const int gx = (t.kind & TILE_GHOST) ? GHOST_X : 0;
-        bool ok = true;
-        if constexpr (TC) {
-            const int warp = tid >> 5, lane = tid & 31;
-            if (lane == 0) {
-                const bool diag = warp >= 4;
-                const int ix = diag ? warp + 1 : warp < 2 ? 1 + 2 * warp : 5 + 2 * warp;
-                mbar_init(&bars[ix - 1], 1);
-                if (!diag) mbar_init(&bars[ix], 1);
-                fence_mbar_init();
-                issue_box<S>(sm + box_start<S>(ix), maps, t.x0, t.y0, gx, TILE_CX, TILE_CY, ix, &bars[ix - 1]);
-                if (!diag)
-                    issue_box<S>(sm + box_start<S>(ix + 1), maps, t.x0, t.y0, gx, TILE_CX, TILE_CY, ix + 1, &bars[ix]);
-            }
-            __syncwarp();
-            const StageView<S> v{stage + gsp->state_off, a.nflags + gsp->node_off, (int)gsp->plane, gsp->pitch};
-            // FP64 has one form of the weights
-            if (sizeof(S) == 8 ? fm != 0 : fm == 1) ok = sweep_warp<S, 1>(t, gsp, v, sm, bars, warp, lane);
-            else if (fm == 2) ok = sweep_warp<S, sizeof(S) == 4 ? 2 : 1>(t, gsp, v, sm, bars, warp, lane);
-            else ok = sweep_warp<S, 0>(t, gsp, v, sm, bars, warp, lane);
-        } else {
-            if (tid == 0) {
-                for (int b = 0; b < a.slots; ++b) mbar_init(&bars[b], 1);
-                fence_mbar_init();
-            }
-            __syncthreads();
-            const StageView<S> v{stage + gsp->state_off, a.nflags + gsp->node_off, (int)gsp->plane, gsp->pitch};
-            for (int i0 = 1, r = 0; i0 <= 12; i0 += a.slots, ++r) {
-                const int nd = min(a.slots, 13 - i0);
-                if (tid == 0) {
-                    fence_proxy_async_smem();
-                    for (int d = 0; d < nd; ++d)
-                        issue_box<S>(sm + d * Lr.slot_pairs, maps, t.x0, t.y0, gx, TX, TY, i0 + d, &bars[d]);
-                }
-                // every thread waits for every copy of the round
-                for (int d = 0; d < nd; ++d) ok = mbar_wait_bounded(&bars[d], r & 1, TMA_WAIT_POLLS) && ok;
-                if (t.kind & TILE_FIX) {
-                    for (int d = 0; d < nd; ++d) {
-                        // x cells, then (they read other cells) y cells: the
-                        // two touch disjoint parts of a box
-                        fix_box<S>(sm + d * Lr.slot_pairs, gsp, v, t, TX, TY, i0 + d, tid, NT);
-                    }
-                    __syncthreads();
-                }
-                S *save = reinterpret_cast<S *>(sm + wall_off);
-                if (sizeof(S) == 8 ? fm != 0 : fm == 1)
-                    sweep_block<S, 1>(t, gsp, sm, Lr.slot_pairs, sm + part_off, save, TX, TY, i0, nd, tid, NT);
-                else if (fm == 2)
-                    sweep_block<S, sizeof(S) == 4 ? 2 : 1>(t, gsp, sm, Lr.slot_pairs, sm + part_off, save, TX, TY, i0, nd,
-                                                           tid, NT);
-                else sweep_block<S, 0>(t, gsp, sm, Lr.slot_pairs, sm + part_off, save, TX, TY, i0, nd, tid, NT);
-                __syncthreads();
-            }
-        }
-        if (!ok) atomicOr(&a.status[t.sample], STATUS_TIMEOUT);
-    }
-    __syncthreads();
-
-    const SampleParams &sp = s_sp;
+    constexpr bool F32 = sizeof(S) == 4, DEV = F32;
+    constexpr bool EARLY = flux_early<S>(MODE);
+    if (!EARLY) __syncthreads();
     const int tx = tid % TX, ty = tid / TX;
     const int x = t.x0 + tx, y = t.y0 + ty;
-    const int o = y * sp.pitch + x;
-    // the node's place in a part array, and the arrays' starts
-    const int pn = ty * PR + tx;
-    V *const parts = sm + part_off;
-    auto part = [&](int i, int axis) -> V & {
-        if constexpr (TC && SWEEP) {
-            if (box_shape(i) == BOX_XY && axis == 0) return parts[(i - 5) * PP + pn];
-            return sm[box_start<S>(i) + pn];
-        } else {
-            return parts[part_index(i, axis) * PP + pn];
-        }
-    };
+    const int o = y * sp.pitch + x, PL = (int)sp.plane;
     bool active = x < sp.nx && y < sp.ny;
     if (active && (!SWEEP || (t.kind & TILE_FIX))) active = (a.nflags[sp.node_off + o] & NF_TYPE) == 0;
-    if (SWEEP && (t.kind & TILE_FIX) && active) {
-        // at a clamped edge cFLUX's upstream face is the node's own (index
-        // clamps): no difference
-        const bool cx = !(sp.flags & SF_PERX), cy = !(sp.flags & SF_PERY);
+    V *__restrict__ st = pair_base(a.state, sp) + o;
+    C kx, ky;  // dt/dx, dt/dy (FP64: times |e|)
+    V fv[NQ];  // the state (after RK3 stage 3: the update's partial sum)
+    auto load = [&]() {
+        const double cs = F32 ? 1.0 : sp.c;
+        kx = (C)__dmul_rn(a.tdx[sp.xoff + x], cs);
+        ky = (C)__dmul_rn(a.tdy[sp.yoff + y], cs);
+        if (EARLY || MODE != 1) {
 #pragma unroll
-        for (int i = 1; i < NQ; ++i) {
-            if (cx && lat_ex(i) != 0 && x == (lat_ex(i) > 0 ? 0 : sp.nx - 1)) part(i, 0) = kc<V>(0.0);
-            if (cy && lat_ey(i) != 0 && y == (lat_ey(i) > 0 ? 0 : sp.ny - 1)) part(i, 1) = kc<V>(0.0);
+            for (int i = 0; i < NQ; ++i) fv[i] = st[i * PL];
         }
-        // straight walls: the factor of the wall node below (above), from the
-        // faces into it that the sweeps kept, and its flux into this node
-        const StageView<S> v{stage + sp.state_off, nullptr, (int)sp.plane, sp.pitch};
-        const double *fr = a.fref + NPL * t.sample;
-        const S *save = reinterpret_cast<const S *>(sm + wall_off);
-        auto wall = [&](int yw, int w, const int (&in)[4], const int (&out)[4]) {
-            const double dd = a.dyv[sp.yoff + yw];
-            double fin = 0, fout = 0;
-            V fs[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                fs[q] = ldv(v, out[q], x, yw);
-                const double ci = sp.c * (lat_ey(in[q]) == 2 || lat_ey(in[q]) == -2 ? 2 : 1);
-                fin = wall_in(fin, save[(4 * w + wall_slot_in(in[q])) * TX + tx], fr[in[q]], ci, dd);
-                fout = wall_out(fout, (double)fs[q].x, fr[out[q]], ci, dd);
-            }
-            const C am1 = a.phased ? a.template alpha_as<C>()[sp.node_off + (long long)yw * sp.pitch + x]
-                                   : (C)wall_ratio_m1(fin, fout);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                V &p = part(out[q], 1);
-                p = xsub(p, wall_flux<C>(am1, fs[q], fr, out[q], face_arg<C>(sp, lat_ey(out[q]))));
-            }
-        };
-        if ((t.kind & TILE_WALLS) && y == 1) wall(0, 0, {4, 7, 8, 12}, {2, 6, 5, 10});
-        if ((t.kind & TILE_WALLN) && y == sp.ny - 2) wall(sp.ny - 1, 1, {2, 5, 6, 10}, {4, 8, 7, 12});
+    };
+    if (EARLY) {
+        if (active) load();
+        __syncthreads();
     }
-    if constexpr (!SWEEP) {
-        if (active) {
-            const StageView<S> v{stage + sp.state_off, a.nflags + sp.node_off, (int)sp.plane, sp.pitch};
-            const S *alpha = a.template alpha_as<S>() + sp.node_off;
-            const double *fr = a.fref + NPL * t.sample;
-#pragma unroll 1
-            for (int i = 1; i < NQ; ++i)
-#pragma unroll 1
-                for (int axis = 0; axis < 2; ++axis) {
-                    const int e = isgn(axis == 0 ? c_EX[i] : c_EY[i]);
-                    if (e == 0) continue;
-                    // upstream face: index(x, -e), reflected at a mirror edge
-                    int m;
-                    const int u = bc_index(sp, axis == 0 ? x : y, -e, axis, m);
-                    const int iu = m ? (axis == 0 ? c_MIR_EW[i] : c_MIR_NS[i]) : i;
-                    const V out = node_face<S>(sp, v, alpha, fr, i, axis, x, y);
-                    const V in = axis == 0 ? node_face<S>(sp, v, alpha, fr, iu, 0, u, y)
-                                           : node_face<S>(sp, v, alpha, fr, iu, 1, x, u);
-                    parts[part_index(i, axis) * PP + pn] = xsub(out, in);
-                }
-        }
-    }
-
     double res_part = 0;
     if (active) {
-        V *__restrict__ st = pair_base(a.state, sp) + o;
-        V *__restrict__ b3 = pair_base(a.buf3, sp) + o;
-        const int PL = (int)sp.plane;
+        const S *stage = MODE == 2 ? a.buf3 : a.buf2;
+        if (SWEEP && (t.kind & TILE_FIX)) {
+            // at a clamped edge cFLUX's upstream face is the node's own (index
+            // clamps): no difference
+            const bool cx = !(sp.flags & SF_PERX), cy = !(sp.flags & SF_PERY);
+#pragma unroll
+            for (int i = 1; i < NQ; ++i) {
+                if (cx && lat_ex(i) != 0 && x == (lat_ex(i) > 0 ? 0 : sp.nx - 1)) part(i, 0) = kc<V>(0.0);
+                if (cy && lat_ey(i) != 0 && y == (lat_ey(i) > 0 ? 0 : sp.ny - 1)) part(i, 1) = kc<V>(0.0);
+            }
+            // straight walls: the factor of the wall node below (above), from
+            // the faces into it that the sweeps kept, and its flux into this node
+            const StageView<S> v{stage + sp.state_off, nullptr, (int)sp.plane, sp.pitch};
+            const double *fr = a.fref + NPL * t.sample;
+            auto wall = [&](int yw, int w, const int (&in)[4], const int (&out)[4]) {
+                const double dd = a.dyv[sp.yoff + yw];
+                double fin = 0, fout = 0;
+                V fs[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    fs[q] = ldv(v, out[q], x, yw);
+                    const double ci = sp.c * (lat_ey(in[q]) == 2 || lat_ey(in[q]) == -2 ? 2 : 1);
+                    fin = wall_in(fin, save[(4 * w + wall_slot_in(in[q])) * TX + tx], fr[in[q]], ci, dd);
+                    fout = wall_out(fout, (double)fs[q].x, fr[out[q]], ci, dd);
+                }
+                const C am1 = a.phased ? a.template alpha_as<C>()[sp.node_off + (long long)yw * sp.pitch + x]
+                                       : (C)wall_ratio_m1(fin, fout);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    V &p = part(out[q], 1);
+                    p = xsub(p, wall_flux<C>(am1, fs[q], fr, out[q], face_arg<C>(sp, lat_ey(out[q]))));
+                }
+            };
+            if ((t.kind & TILE_WALLS) && y == 1) wall(0, 0, {4, 7, 8, 12}, {2, 6, 5, 10});
+            if ((t.kind & TILE_WALLN) && y == sp.ny - 2) wall(sp.ny - 1, 1, {2, 5, 6, 10}, {4, 8, 7, 12});
+        }
+        if (!EARLY) load();
         // divergence dt (F_out - F_in)/dx of direction i (cFLUX,
         // cpuLBM.cpp:1436-1470): the parts times dt/dx and dt/dy (FP64: and |e|)
-        constexpr bool F32 = sizeof(S) == 4;
-        const double cs = F32 ? 1.0 : sp.c;
-        const C kx = (C)__dmul_rn(a.tdx[sp.xoff + x], cs), ky = (C)__dmul_rn(a.tdy[sp.yoff + y], cs);
         auto div = [&](int i) -> V {
             const C ux = F32 || lat_ex(i) % 2 ? kx : kx + kx, uy = F32 || lat_ey(i) % 2 ? ky : ky + ky;
             const V vx = make_pair2(ux, ux), vy = make_pair2(uy, uy);
@@ -600,23 +553,21 @@ k_flux(KArgs<S> a)
             if (box_shape(i) == BOX_Y) return xmul(vy, part(i, 1));
             return xfma(vy, part(i, 1), xmul(vx, part(i, 0)));
         };
-        constexpr bool DEV = sizeof(S) == 4;
         bool bad = false, bad_eq = false;
-        MomentSums ms;       // of the new state, when the residual is wanted
+        MomentSums ms;           // of the new state, when the residual is wanted
         S fin_r = 0, fin_h = 0;  // NaN / Inf propagate through these sums as through FP64 ones
         if constexpr (MODE == 1) {
             // RK3 stage 3 (cpuLBM.cpp:1928-1993) and the part of the update
             // (cpuLBM.cpp:1999-2042) that does not need the stage-3 fluxes
-            const int gd = ghost_offset(sp, x);
-            V fv[NQ];
-#pragma unroll
-            for (int i = 0; i < NQ; ++i) fv[i] = st[i * PL];
+            const V *__restrict__ b2 = pair_base(a.buf2, sp) + o;
+            V *__restrict__ b3 = pair_base(a.buf3, sp) + o;
             // stage-1 moments (= stage 2's) and the moments of f - div F(f2)
             // (macroProp3, cpuLBM.cpp:973-1032)
             MomentSums s1, s3;
 #pragma unroll
             for (int i = 0; i < NQ; ++i) {
-                const double f = (double)fv[i].x, h = (double)fv[i].y;
+                const V v = EARLY ? fv[i] : st[i * PL];
+                const double f = (double)v.x, h = (double)v.y;
                 s1.add(i, f, h);
                 const V D = div(i);
                 s3.add(i, i ? __dsub_rn(f, (double)D.x) : f, i ? __dsub_rn(h, (double)D.y) : h);
@@ -626,44 +577,68 @@ k_flux(KArgs<S> a)
             const EqArgs<C, DEV> q3(m3.rho, m3.ux, m3.uy, m3.T, sp);
             const Stage3<C> s(m1, m3, sp);
             double sf3 = 0;
-            auto family = [&](const int fam) {
-                C e1f[4], e1h[4], e3f[4], e3h[4];
-                q1.fam(fam, e1f, e1h);
-                q3.fam(fam, e3f, e3h);
+            // family by family; the state is loaded a second time rather than
+            // kept (13 pairs of registers, which FP64 spilled and FP32 needs
+            // for the loads ahead)
+            V gv[4], g2[4];
+            auto fetch = [&](const int fam) {
                 const int i0 = fam == 0 ? 0 : 4 * fam - 3, n = fam == 0 ? 1 : 4;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < n) {
+                        gv[k] = load_again(st + (i0 + k) * PL);
+                        if (F32) g2[k] = b2[(i0 + k) * PL];
+                    }
+            };
+            auto family = [&](const int fam) {
+                const int i0 = fam == 0 ? 0 : 4 * fam - 3, n = fam == 0 ? 1 : 4;
+                V hv[4], d2[4];
+                fetch(fam);
+                {
+                    C ef[4], eh[4];
+                    q1.fam(fam, ef, eh);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (k < n) {
+                            hv[k] = gv[k];
+                            d2[k] = s.dist(i0 + k, make_pair2(ef[k], eh[k]), hv[k], F32 ? g2[k] : kc<V>(0.0));
+                        }
+                }
+                C ef[4], eh[4];
+                q3.fam(fam, ef, eh);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (k >= n) break;
                     const int i = i0 + k;
-                    sf3 += (double)e3f[k];
+                    sf3 += (double)ef[k];
                     V n3, acc;
-                    s.update(i, fv[i], div(i), make_pair2(e1f[k], e1h[k]), make_pair2(e3f[k], e3h[k]), n3, acc);
+                    s.update(i, hv[k], div(i), d2[k], make_pair2(ef[k], eh[k]), n3, acc);
                     b3[i * PL] = n3;
-                    if (gd) b3[i * PL + gd] = n3;
                     st[i * PL] = acc;
                 }
             };
 #pragma unroll
             for (int fam = 0; fam < 4; ++fam) family(fam);
+            // the images of nodes near a periodic edge, read back by the few
+            // threads that have one (a store in the loop above would cost
+            // every thread its predicate)
+            if (const int gd = ghost_offset(sp, x)) {
+#pragma unroll 1
+                for (int i = 0; i < NQ; ++i) b3[i * PL + gd] = b3[i * PL];
+            }
             bad_eq = fabs(sf3 - (m3.rho - sp.rho0)) > a.eq_tol * (sizeof(C) == 8 ? 1.0 : fmax(1.0, fabs(m3.rho)));
         } else if constexpr (MODE == 2) {
             // final RK3 combination (cpuLBM.cpp:1999-2042): f = acc - D3/2
-            V acc[NQ];
-#pragma unroll
-            for (int i = 0; i < NQ; ++i) acc[i] = st[i * PL];
 #pragma unroll
             for (int i = 0; i < NQ; ++i) {
-                const V n = i ? xfma(kc<V>(-0.5), div(i), acc[i]) : acc[i];
-                st[i * PL] = n;
+                const V n = i ? xfma(kc<V>(-0.5), div(i), fv[i]) : fv[i];
+                if (i) st[i * PL] = n;
                 fin_r += n.x;
                 fin_h += n.y;
                 if (a.want_residual) ms.add(i, (double)n.x, (double)n.y);
             }
         } else {
             // RK1 update (cpuLBM.cpp:1674-1710), EULER (:2130-2168), EULER_EQ (:2220-2258)
-            V fv[NQ];
-#pragma unroll
-            for (int i = 0; i < NQ; ++i) fv[i] = st[i * PL];
             const Macro m = node_macro_rd([&](int i) { return fv[i]; }, sp);
             const EqArgs<C, DEV> q(m.rho, m.ux, m.uy, m.T, sp);
             const Update<C, MODE> u(m, sp);
@@ -718,16 +693,140 @@ k_flux(KArgs<S> a)
     }
 }
 
+// blocks per SM that the registers leave room for
+template <class S, int MODE, bool SWEEP>
+struct FluxBlocks {
+    static constexpr int value = !SWEEP || sizeof(S) == 8 ? 2 : MODE == 1 ? 2 : 3;
+};
+
+// MODE: 1 = RK3 stage 3 (fluxes of buffer 2), 2 = RK3 final (buffer 3),
+// 3 = RK1 update, 4 = EULER update, 5 = EULER_EQ update (buffer 2)
+// PATH: FLUX_SWEEP or FLUX_GENERAL, the tiles of one kind per launch (a
+// block given the other kind returns at once).
+// TC: the default tile shape, compiled in; other shapes are read from the
+// arguments and give every node the same bits.
+template <class S, int MODE, int PATH, bool TC>
+__global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP && TC>::value) k_flux(KArgs<S> a)
+{
+    using V = Pair<S>;
+    extern __shared__ __align__(128) unsigned char smem_dyn[];
+    __shared__ double red[32];
+    __shared__ SampleParams s_sp;  // kept out of registers: read as needed
+    __shared__ Tile s_tile;
+    constexpr bool SWEEP = PATH == FLUX_SWEEP;
+    const int TX = TC ? TILE_CX : a.tx, TY = TC ? TILE_CY : a.ty, NT = TX * TY;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    V *sm = reinterpret_cast<V *>(smem_dyn + ((128 - (smem_u32(smem_dyn) & 127)) & 127));
+    const Tile t = a.tiles[blockIdx.x];
+    if (tile_sweep(t) != SWEEP) return;
+    constexpr int PH = MODE == 2 ? 2 : 1;
+    const CUtensorMap *maps = a.tmaps + MAPS_PER_SAMPLE * t.sample + (PH == 1 ? 0 : 3);
+    const S *stage = PH == 1 ? a.buf2 : a.buf3;
+    const int PR = TX + 1, PP = part_pairs(TX, TY);
+    constexpr FluxSmem LC = flux_smem<S>(TILE_CX, TILE_CY, true, true, 12);
+    FluxSmem L = LC;
+    if constexpr (!TC) L = flux_smem<S>(TX, TY, false, SWEEP, SWEEP ? a.slots : 0);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + L.bar_off);
+    S *save = reinterpret_cast<S *>(sm + L.wall_off);
+
+    if constexpr (TC && SWEEP) {
+        // each warp asks for its own boxes, and alone waits for them
+        if (lane == 0) {
+            const int ix = warp >= 4 ? warp + 1 : warp < 2 ? 1 + 2 * warp : 5 + 2 * warp;
+            mbar_init(&bars[ix - 1], 1);
+            if (warp < 4) mbar_init(&bars[ix], 1);
+            fence_mbar_init();
+            issue_warp<S>(t, maps, sm, bars, warp);
+        }
+    } else if constexpr (SWEEP) {
+        if (tid == 0) {
+            for (int b = 0; b < a.slots; ++b) mbar_init(&bars[b], 1);
+            fence_mbar_init();
+        }
+    }
+    {
+        const SampleParams *gsp = a.samples + t.sample;
+        for (int k = tid; k < (int)(sizeof(SampleParams) / 4); k += NT)
+            reinterpret_cast<int *>(&s_sp)[k] = reinterpret_cast<const int *>(gsp)[k];
+        if (tid == 0) s_tile = t;
+    }
+    // (what a plain tile's sweeps need is in the tile itself)
+    if (!TC || !SWEEP || flux_early<S>(MODE) || (t.kind & TILE_FIX)) __syncthreads();
+    const SampleParams &sp = s_sp;
+    bool ok = true;
+    if constexpr (TC && SWEEP) {
+        // the rows of the state that the per-node half will read, into L2
+        // (3 % of an FP64 step; FP32 gains nothing)
+        if constexpr (sizeof(S) == 8) {
+            const V *p = pair_base(a.state, sp) + (t.y0 + warp) * sp.pitch + t.x0 + lane;
+            if ((lane & 7) == 0 && t.y0 + warp < sp.ny)
+                for (int i = 0; i < NQ; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i * (int)sp.plane));
+        }
+        ok = sweep_tile<S>(t, sp, stage, sm, save, bars, 0, warp, lane);
+    } else if constexpr (SWEEP) {
+        const int fm = tile_fm(t.kind), gx = (t.kind & TILE_GHOST) ? GHOST_X : 0;
+        for (int i0 = 1, r = 0; i0 <= 12; i0 += a.slots, ++r) {
+            const int nd = min(a.slots, 13 - i0);
+            if (tid == 0) {
+                fence_proxy_async_smem();
+                for (int d = 0; d < nd; ++d)
+                    issue_box<S>(sm + d * L.slot_pairs, maps, t.x0, t.y0, gx, TX, TY, i0 + d, &bars[d]);
+            }
+            // every thread waits for every copy of the round
+            for (int d = 0; d < nd; ++d) ok = mbar_wait_bounded(&bars[d], r & 1, TMA_WAIT_POLLS) && ok;
+            if (t.kind & TILE_FIX) {
+                for (int d = 0; d < nd; ++d) fix_box<S>(sm + d * L.slot_pairs, sp, stage, t, TX, TY, i0 + d, tid, NT);
+                __syncthreads();
+            }
+            V *parts = sm + L.part_off;
+            if (sizeof(S) == 8 ? fm != 0 : fm == 1)
+                sweep_block<S, 1>(t, sp, sm, L.slot_pairs, parts, save, TX, TY, i0, nd, tid, NT);
+            else if (fm == 2)
+                sweep_block<S, sizeof(S) == 4 ? 2 : 1>(t, sp, sm, L.slot_pairs, parts, save, TX, TY, i0, nd, tid, NT);
+            else sweep_block<S, 0>(t, sp, sm, L.slot_pairs, parts, save, TX, TY, i0, nd, tid, NT);
+            __syncthreads();
+        }
+    }
+    if (!ok) atomicOr(&a.status[a.tiles[blockIdx.x].sample], STATUS_TIMEOUT);
+    const int tx = tid % TX, ty = tid / TX;
+    const NodeParts<S, TC && SWEEP> part{TC && SWEEP ? sm : sm + L.part_off, ty * PR + tx, PP};
+    if constexpr (!SWEEP) {
+        const int x = t.x0 + tx, y = t.y0 + ty;
+        if (x < sp.nx && y < sp.ny && (a.nflags[sp.node_off + y * sp.pitch + x] & NF_TYPE) == 0) {
+            const StageView<S> v{stage + sp.state_off, a.nflags + sp.node_off, (int)sp.plane, sp.pitch};
+            const S *alpha = a.template alpha_as<S>() + sp.node_off;
+            const double *fr = a.fref + NPL * t.sample;
+#pragma unroll 1
+            for (int i = 1; i < NQ; ++i)
+#pragma unroll 1
+                for (int axis = 0; axis < 2; ++axis) {
+                    const int e = isgn(axis == 0 ? c_EX[i] : c_EY[i]);
+                    if (e == 0) continue;
+                    // upstream face: index(x, -e), reflected at a mirror edge
+                    int m;
+                    const int u = bc_index(sp, axis == 0 ? x : y, -e, axis, m);
+                    const int iu = m ? (axis == 0 ? c_MIR_EW[i] : c_MIR_NS[i]) : i;
+                    const V out = node_face<S>(sp, v, alpha, fr, i, axis, x, y);
+                    const V in = axis == 0 ? node_face<S>(sp, v, alpha, fr, iu, 0, u, y)
+                                           : node_face<S>(sp, v, alpha, fr, iu, 1, x, u);
+                    part(i, axis) = xsub(out, in);
+                }
+        }
+    }
+    node_phase<S, MODE, SWEEP>(a, s_tile, sp, part, save, red, TX, NT, tid);
+}
+
 // ----------------------------------------------------------------- launchers
-template <class S, int PATH, bool TC>
-void launch_flux_t(int mode, const KArgs<S> &k, int ntiles, int NT, size_t sm, cudaStream_t st)
+// calls f with the mode as a compile-time value
+template <class F>
+void with_mode(int mode, F f)
 {
     switch (mode) {
-    case 1: k_flux<S, 1, PATH, TC><<<ntiles, NT, sm, st>>>(k); break;
-    case 2: k_flux<S, 2, PATH, TC><<<ntiles, NT, sm, st>>>(k); break;
-    case 3: k_flux<S, 3, PATH, TC><<<ntiles, NT, sm, st>>>(k); break;
-    case 4: k_flux<S, 4, PATH, TC><<<ntiles, NT, sm, st>>>(k); break;
-    default: k_flux<S, 5, PATH, TC><<<ntiles, NT, sm, st>>>(k); break;
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    default: f(std::integral_constant<int, 5>()); break;
     }
 }
 
@@ -739,12 +838,12 @@ cudaError_t launch_flux(int mode, const KArgs<S> &a, int ntiles, int path, cudaS
     k.slots = def ? 12 : flux_slots<S>(k.tx, k.ty);
     const int NT = k.tx * k.ty;
     const size_t sm = flux_smem_bytes_t<S>(k.tx, k.ty, sweep);
-    if (sweep) {
-        if (def) launch_flux_t<S, FLUX_SWEEP, true>(mode, k, ntiles, NT, sm, st);
-        else launch_flux_t<S, FLUX_SWEEP, false>(mode, k, ntiles, NT, sm, st);
-    } else {
-        launch_flux_t<S, FLUX_GENERAL, false>(mode, k, ntiles, NT, sm, st);
-    }
+    with_mode(mode, [&](auto m) {
+        constexpr int M = decltype(m)::value;
+        if (!sweep) k_flux<S, M, FLUX_GENERAL, false><<<ntiles, NT, sm, st>>>(k);
+        else if (!def) k_flux<S, M, FLUX_SWEEP, false><<<ntiles, NT, sm, st>>>(k);
+        else k_flux<S, M, FLUX_SWEEP, true><<<ntiles, NT, sm, st>>>(k);
+    });
     return cudaGetLastError();
 }
 
@@ -753,14 +852,16 @@ cudaError_t prepare_flux()
 {
     const int maxsm = 224 * 1024;
     cudaError_t e = cudaSuccess;
-#define UQ_FLUX_SMEM1(M, P, T)                                                                             \
-    if (e == cudaSuccess)                                                                                  \
-        e = cudaFuncSetAttribute(k_flux<S, M, P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm);
-#define UQ_FLUX_SMEM(M) \
-    UQ_FLUX_SMEM1(M, FLUX_SWEEP, true) UQ_FLUX_SMEM1(M, FLUX_SWEEP, false) UQ_FLUX_SMEM1(M, FLUX_GENERAL, false)
-    UQ_FLUX_SMEM(1) UQ_FLUX_SMEM(2) UQ_FLUX_SMEM(3) UQ_FLUX_SMEM(4) UQ_FLUX_SMEM(5)
-#undef UQ_FLUX_SMEM
-#undef UQ_FLUX_SMEM1
+    auto allow = [&](auto *kernel) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm);
+    };
+    for (int mode = 1; mode <= 5; ++mode)
+        with_mode(mode, [&](auto m) {
+            constexpr int M = decltype(m)::value;
+            allow(k_flux<S, M, FLUX_GENERAL, false>);
+            allow(k_flux<S, M, FLUX_SWEEP, false>);
+            allow(k_flux<S, M, FLUX_SWEEP, true>);
+        });
     return e;
 }
 

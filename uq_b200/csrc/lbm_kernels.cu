@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256, Stage0Blocks<S>::value) k_stage0(KArgs<S>
             if (k >= n) break;
             const int i = i0 + k;
             sf += (double)fe[k];
-            const V nv = p.value(i, v[i], make_pair2(fe[k], he[k]));
+                        const V nv = p.value(i, v[i], make_pair2(fe[k], he[k]));
             b2[i * PL] = nv;
             if (gd) b2[i * PL + gd] = nv;
         }

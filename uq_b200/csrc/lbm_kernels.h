@@ -17,7 +17,7 @@ constexpr int STATUS_NONFINITE = 2;  // NaN / Inf / rho <= 0 in the state
 constexpr int STATUS_TIMEOUT = 4;    // a bounded device-side wait ran out
 
 // tensor maps per sample: the stage buffers 2 and 3, each with the stencil
-// kernels' three box shapes (x lines, y lines, both; see lbm_flux.cuh)
+// kernels' three box shapes (x lines, y lines, both; see lbm_box.h)
 constexpr int MAPS_PER_SAMPLE = 6;
 // the default tile shape, also compiled into the stencil kernels (box
 // widths, strides and the thread-to-line map become constants); other shapes

@@ -252,9 +252,8 @@ static lbm_status step_noalloc(const lbm_config *cfg, int Nx, int Ny, const int 
     sp.ntile = (int)tiles.size();
 
     CUtensorMap maps[MAPS_PER_SAMPLE];
-    for (int b = 0; b < MAPS_PER_SAMPLE; ++b)
-        if (!encode_box_map(encoder(), true, sp, base + (b < 3 ? NA_OFF_BUF2 : NA_OFF_BUF3), b % 3, NA_TX, NA_TY, &maps[b]))
-            throw LbmError(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    if (!encode_box_maps(encoder(), true, sp, base + NA_OFF_BUF2, base + NA_OFF_BUF3, NA_TX, NA_TY, maps))
+        throw LbmError(LBM_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     // small host-to-device copies of values on this stack frame (staged by
     // the driver before the call returns)
     CU(cudaMemcpyAsync(base + NA_OFF_SP, &sp, sizeof(sp), cudaMemcpyHostToDevice, st));

@@ -19,6 +19,20 @@ __device__ __forceinline__ const Pair<S> *pair_base(const S *base, const SampleP
     return reinterpret_cast<const Pair<S> *>(base + sp.state_off);
 }
 
+// a second load of a value that was loaded before, not its register kept
+__device__ __forceinline__ float2 load_again(const float2 *p)
+{
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double2 load_again(const double2 *p)
+{
+    double2 v;
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+
 // Ghost columns (SampleParams::gx): a node within gx of an x edge also
 // stores its stage-buffer values at its periodic image beyond the other
 // edge.  The offset of that image (0: none) for the node at x; a stage value
@@ -183,16 +197,17 @@ struct PointStage<double, RK> {
 // (cpuLBM.cpp:1999-2042) that does not need the stage-3 fluxes, of direction
 // i: from the state v, the divergence D of stage 2's fluxes, and the
 // equilibria at stage 1's (= 2's) and stage 3's moments, the stage value n3
-// and the partial update acc.  Stage 2's value is formed again from v.
+// and the partial update acc.  f2: stage 2's value (FP32; FP64 relaxes from v).
 template <class C>
 struct Stage3;
 template <>
 struct Stage3<float> {
-    PointStage<float, 1> p;
     float2 A2, A3;
-    float hdt, cu3, cv3, g2, g3, ia3, ib3;
-    __device__ __forceinline__ Stage3(const Macro &m1, const Macro &m3, const SampleParams &sp) : p(m1, sp)
+    float hdt, cu1, cv1, cu3, cv3, g2, g3, ia3, ib3;
+    __device__ __forceinline__ Stage3(const Macro &m1, const Macro &m3, const SampleParams &sp)
     {
+        cu1 = xmul((float)sp.c, (float)m1.ux);
+        cv1 = xmul((float)sp.c, (float)m1.uy);
         const float rq1 = (float)m1.q, rq3 = (float)m3.q, Pr = (float)sp.Pr;
         hdt = xmul((float)sp.dt, 0.5f);
         cu3 = xmul((float)sp.c, (float)m3.ux);
@@ -205,10 +220,11 @@ struct Stage3<float> {
         ia3 = __fdiv_rn(1.f, xadd(1.f, A3.x));
         ib3 = __fdiv_rn(1.f, xadd(1.f, A3.y));
     }
-    __device__ __forceinline__ void update(int i, float2 v, float2 D, float2 e1, float2 e3, float2 &n3, float2 &acc) const
+    // the distance of stage 2 from its equilibrium
+    __device__ __forceinline__ float2 dist(int, float2 e1, float2, float2 f2) const { return xsub(e1, f2); }
+    __device__ __forceinline__ void update(int i, float2 v, float2 D, float2 D1, float2 e3, float2 &n3, float2 &acc) const
     {
-        const float2 D1 = xsub(e1, p.value(i, v, e1));
-        const float eu2 = e_dot<float>(i, p.cu, p.cv), eu3 = e_dot<float>(i, cu3, cv3);
+        const float eu2 = e_dot<float>(i, cu1, cv1), eu3 = e_dot<float>(i, cu3, cv3);
         const float2 X = xfma(A2, D1, xfma(A3, e3, i ? xsub(v, D) : v));
         const float f3 = xmul(X.x, ia3);
         // hdt times the coupling term
@@ -223,10 +239,14 @@ struct Stage3<double> {
     Relax64 r1, r3;
     __device__ __forceinline__ Stage3(const Macro &m1, const Macro &m3, const SampleParams &sp)
         : r1(m1, sp, 0.5), r3(m3, sp, 0.5) {}
-    __device__ __forceinline__ void update(int i, double2 v, double2 D, double2 e1, double2 e3, double2 &n3,
+    __device__ __forceinline__ double2 dist(int i, double2 e1, double2 v, double2) const
+    {
+        return r1.stage2(i, xsub(e1, v));
+    }
+    __device__ __forceinline__ void update(int i, double2 v, double2 D, double2 d2, double2 e3, double2 &n3,
                                            double2 &acc) const
     {
-        const double2 d2 = r1.stage2(i, xsub(e1, v)), S2 = xmul(r1.c, d2);  // e - f2; dt/2 (e - f2)/tau
+        const double2 S2 = xmul(r1.c, d2);  // dt/2 (e - f2)/tau
         const double s2h = xmul(r1.coupling(i), d2.x);
         // Y: what f3 relaxes from
         double2 Y = xadd(i ? xsub(v, D) : v, S2);
