@@ -46,6 +46,7 @@ struct SampleParams {
     long long state_off; // element offset of plane 0 in every state buffer (even)
     long long plane;     // nodes per plane
     long long node_off;  // offset into per-node arrays
+    long long lat_off;   // nodes (nx ny each) of the samples before, in a batch
     int xoff, yoff;      // offsets into the per-column / per-row spacing tables
     double R, bR, K, Tc, inv_sRTc, RTc, mu, Pr, dt, c;
     // Reference rest state of the stored deviations (mixed path): the state

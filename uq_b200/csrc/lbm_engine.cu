@@ -649,6 +649,7 @@ struct lbm_batch {
             SampleParams p = ps.p;
             p.state_off = state_off + (p.gx ? GHOST_SLACK : 0);  // the first row's left ghosts before it
             p.node_off = node_off;
+            p.lat_off = lattice_nodes;
             p.xoff = (int)v_tdx.size();
             p.yoff = (int)v_tdy.size();
             fref_host.insert(fref_host.end(), ps.fref, ps.fref + NPL);
@@ -809,29 +810,38 @@ struct lbm_batch {
         const double *src[4] = {rho, ux, uy, T};
         for (int k = 0; k < 4; ++k)
             CU(cudaMemcpyAsync(scratch.p + k * n, src[k], n * sizeof(double), cudaMemcpyHostToDevice, stream));
+        write_fields(s, 1, scratch.p, n, n);
+    }
+
+    // the state of samples s0 .. s0 + ns - 1 from fields on the device,
+    // `stride` values apart (`nodes`: the most nodes of one)
+    void write_fields(int s0, int ns, const double *fields, long long stride, long long nodes)
+    {
         if (prec == LBM_PREC_F64)
-            CU(launch_set_macro<double>(d_sp.p, s, reinterpret_cast<double *>(state.p), reinterpret_cast<double *>(buf2.p),
-                                        reinterpret_cast<double *>(buf3.p), scratch.p, nflags.p, d_fref.p, n, stream));
+            CU(launch_set_macro<double>(d_sp.p, s0, ns, reinterpret_cast<double *>(state.p),
+                                        reinterpret_cast<double *>(buf2.p), reinterpret_cast<double *>(buf3.p), fields,
+                                        stride, nflags.p, d_fref.p, nodes, stream));
         else
-            CU(launch_set_macro<float>(d_sp.p, s, reinterpret_cast<float *>(state.p), reinterpret_cast<float *>(buf2.p),
-                                       reinterpret_cast<float *>(buf3.p), scratch.p, nflags.p, d_fref.p, n, stream));
-        fill_ghosts(s, 1);
+            CU(launch_set_macro<float>(d_sp.p, s0, ns, reinterpret_cast<float *>(state.p),
+                                       reinterpret_cast<float *>(buf2.p), reinterpret_cast<float *>(buf3.p), fields,
+                                       stride, nflags.p, d_fref.p, nodes, stream));
+        fill_ghosts(s0, ns);
+    }
+    // and the fields from the state
+    void read_fields(int s0, int ns, double *out, long long stride, long long nodes)
+    {
+        if (prec == LBM_PREC_F64)
+            CU(launch_macro_out<double>(d_sp.p, s0, ns, reinterpret_cast<double *>(state.p), out, stride, nodes, stream));
+        else
+            CU(launch_macro_out<float>(d_sp.p, s0, ns, reinterpret_cast<float *>(state.p), out, stride, nodes, stream));
     }
 
     // all samples' fields in one device buffer (5 fields x lattice nodes,
     // made on first use): per field one copy to or from the host
     DevBuf<double> all_fields;
-    std::vector<long long> lattice_off;  // per sample: first value in the concatenated fields
 
     void ensure_all_fields()
     {
-        if (lattice_off.empty()) {
-            long long off = 0;
-            for (const HostSample &h : hs) {
-                lattice_off.push_back(off);
-                off += (long long)h.nx * h.ny;
-            }
-        }
         if (all_fields.n < (size_t)(5 * lattice_nodes)) all_fields.alloc(5 * lattice_nodes);
     }
 
@@ -842,36 +852,13 @@ struct lbm_batch {
         for (int k = 0; k < 4; ++k)
             CU(cudaMemcpyAsync(all_fields.p + k * lattice_nodes, src[k], lattice_nodes * sizeof(double),
                                cudaMemcpyHostToDevice, stream));
-        for (size_t s = 0; s < hs.size(); ++s) {
-            const long long n = (long long)hs[s].nx * hs[s].ny;
-            // the four fields of sample s, each n values, lattice_nodes apart
-            double *f0 = all_fields.p + lattice_off[s];
-            if (prec == LBM_PREC_F64)
-                CU(launch_set_macro_strided<double>(d_sp.p, (int)s, reinterpret_cast<double *>(state.p),
-                                                    reinterpret_cast<double *>(buf2.p),
-                                                    reinterpret_cast<double *>(buf3.p), f0, lattice_nodes, nflags.p,
-                                                    d_fref.p, n, stream));
-            else
-                CU(launch_set_macro_strided<float>(d_sp.p, (int)s, reinterpret_cast<float *>(state.p),
-                                                   reinterpret_cast<float *>(buf2.p), reinterpret_cast<float *>(buf3.p),
-                                                   f0, lattice_nodes, nflags.p, d_fref.p, n, stream));
-        }
-        fill_ghosts(0, (int)hs.size());
+        write_fields(0, (int)hs.size(), all_fields.p, lattice_nodes, (long long)max_nodes);
     }
 
     void get_macro_all(double *rho, double *ux, double *uy, double *T, double *p)
     {
         ensure_all_fields();
-        for (size_t s = 0; s < hs.size(); ++s) {
-            const long long n = (long long)hs[s].nx * hs[s].ny;
-            double *out = all_fields.p + lattice_off[s];
-            if (prec == LBM_PREC_F64)
-                CU(launch_macro_out_strided<double>(d_sp.p, (int)s, reinterpret_cast<double *>(state.p), out,
-                                                    lattice_nodes, n, stream));
-            else
-                CU(launch_macro_out_strided<float>(d_sp.p, (int)s, reinterpret_cast<float *>(state.p), out,
-                                                   lattice_nodes, n, stream));
-        }
+        read_fields(0, (int)hs.size(), all_fields.p, lattice_nodes, (long long)max_nodes);
         double *dst[5] = {rho, ux, uy, T, p};
         for (int k = 0; k < 5; ++k)
             if (dst[k])
@@ -936,10 +923,7 @@ struct lbm_batch {
     void get_macro(int s, double *rho, double *ux, double *uy, double *T, double *p)
     {
         const long long n = (long long)hs[s].nx * hs[s].ny;
-        if (prec == LBM_PREC_F64)
-            CU(launch_macro_out<double>(d_sp.p, s, reinterpret_cast<double *>(state.p), scratch.p, n, stream));
-        else
-            CU(launch_macro_out<float>(d_sp.p, s, reinterpret_cast<float *>(state.p), scratch.p, n, stream));
+        read_fields(s, 1, scratch.p, n, n);
         double *dst[5] = {rho, ux, uy, T, p};
         for (int k = 0; k < 5; ++k)
             if (dst[k]) CU(cudaMemcpyAsync(dst[k], scratch.p + k * n, n * sizeof(double), cudaMemcpyDeviceToHost, stream));

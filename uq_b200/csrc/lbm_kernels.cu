@@ -188,97 +188,164 @@ __global__ void k_residual(const SampleParams *samples, int nsamples, const doub
 }
 
 // ------------------------------------------------------------ boundary I/O
-// macroPropShort for every node of one sample, written in the reference's
-// [x*Ny + y] order: rho, ux, uy, T, p, each `stride` values apart.
-template <class S>
-__global__ void k_macro_out(const SampleParams *samples, int s, const S *state, double *out, long long stride)
+// Fields at the boundary are in the reference's [x*Ny + y] order, y fastest;
+// the planes have x fastest.  A block moves tiles of 32 columns x 8 rows
+// through shared memory, so that both sides are read and written in whole
+// sectors (8 values along y are 64 bytes; a thread per boundary value touched
+// a sector of every plane for 8 bytes of it).  Blocks (., j) take sample
+// s0 + j; with `all`, a sample's fields start SampleParams::lat_off values in.
+constexpr int IO_X = 32, IO_Y = 8, IO_N = IO_X * IO_Y;
+
+template <class F>
+__device__ __forceinline__ void io_tiles(const SampleParams &sp, F f)
 {
-    const SampleParams sp = samples[s];
-    const long long n = (long long)sp.nx * sp.ny;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const int y = (int)(k % sp.ny), x = (int)(k / sp.ny);
-        const Macro m = node_macro<S>(pair_base(state, sp), sp, (long long)y * sp.pitch + x);
-        out[k] = m.rho;
-        out[stride + k] = m.ux;
-        out[2 * stride + k] = m.uy;
-        out[3 * stride + k] = m.T;
-        out[4 * stride + k] = m.p;
-    }
+    const int ntx = (sp.nx + IO_X - 1) / IO_X, nt = ntx * ((sp.ny + IO_Y - 1) / IO_Y);
+    for (int q = blockIdx.x; q < nt; q += gridDim.x) f(q % ntx * IO_X, q / ntx * IO_Y);
 }
 
-// planes <-> reference AoS [(x*Ny + y)*13 + i] in FP64
+// macroPropShort of every node: rho, ux, uy, T, p, each `stride` values apart
 template <class S>
-__global__ void k_dist_io(const SampleParams *samples, int s, S *state, S *buf2, S *buf3, double *aos, int to_aos,
-                          const uint8_t *nflags, const double *fref)
+__global__ void __launch_bounds__(IO_N) k_macro_out(const SampleParams *samples, int s0, int all, const S *state, double *out,
+                                                    long long stride)
 {
-    const double *fr = fref + NPL * s;
-    const SampleParams sp = samples[s];
-    const long long n = (long long)sp.nx * sp.ny * NQ;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(k % NQ);
-        const long long xy = k / NQ;
-        const int y = (int)(xy % sp.ny), x = (int)(xy / sp.ny);
-        const long long o = (long long)y * sp.pitch + x;
-        const long long e = (long long)i * sp.plane + o;
-        if (to_aos) {
-            const Pair<S> v = pair_base(state, sp)[e];
-            aos[k] = (double)v.x + fr[i];
-            aos[n + k] = (double)v.y + fr[NQ + i];
-        } else {
-            const Pair<S> v = make_pair2((S)(aos[k] - fr[i]), (S)(aos[n + k] - fr[NQ + i]));
-            pair_base(state, sp)[e] = v;
-            if (nflags[sp.node_off + o] & NF_TYPE) {  // fixed nodes seed the stage buffers
-                pair_base(buf2, sp)[e] = v;
-                pair_base(buf3, sp)[e] = v;
+    __shared__ double buf[5][IO_Y][IO_X + 1];
+    const SampleParams &sp = samples[s0 + blockIdx.y];
+    const int t = threadIdx.x;
+    if (all) out += sp.lat_off;
+    io_tiles(sp, [&](int x0, int y0) {
+        {
+            const int lx = t % IO_X, ly = t / IO_X, x = x0 + lx, y = y0 + ly;
+            if (x < sp.nx && y < sp.ny) {
+                const Macro m = node_macro<S>(pair_base(state, sp), sp, (long long)y * sp.pitch + x);
+                const double v[5] = {m.rho, m.ux, m.uy, m.T, m.p};
+#pragma unroll
+                for (int k = 0; k < 5; ++k) buf[k][ly][lx] = v[k];
             }
         }
-    }
+        __syncthreads();
+        const int lx = t / IO_Y, ly = t % IO_Y, x = x0 + lx, y = y0 + ly;
+        if (x < sp.nx && y < sp.ny) {
+#pragma unroll
+            for (int k = 0; k < 5; ++k) out[k * stride + (long long)x * sp.ny + y] = buf[k][ly][lx];
+        }
+        __syncthreads();
+    });
 }
 
-// f, h = equilibria of per-node fields given in [x*Ny + y] order (FP64):
-// rho, ux, uy, T, each `stride` values apart
+// planes <-> reference AoS [(x*Ny + y)*13 + i] in FP64, f then h, of sample s
 template <class S>
-__global__ void k_set_macro(const SampleParams *samples, int s, S *state, S *buf2, S *buf3, const double *fields,
-                            long long stride, const uint8_t *nflags, const double *fref)
+__global__ void __launch_bounds__(IO_N) k_dist_io(const SampleParams *samples, int s, S *state, S *buf2, S *buf3, double *aos,
+                                                  int to_aos, const uint8_t *nflags, const double *fref)
 {
+    __shared__ double buf[IO_X][IO_Y * NQ + 1];
     const double *fr = fref + NPL * s;
-    const SampleParams sp = samples[s];
-    const long long n = (long long)sp.nx * sp.ny;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const int y = (int)(k % sp.ny), x = (int)(k / sp.ny);
+    const SampleParams &sp = samples[s];
+    const long long n = (long long)sp.nx * sp.ny * NQ;
+    const int t = threadIdx.x, lx = t % IO_X, ly = t / IO_X;
+    io_tiles(sp, [&](int x0, int y0) {
+        const int x = x0 + lx, y = y0 + ly;
+        const bool in = x < sp.nx && y < sp.ny;
         const long long o = (long long)y * sp.pitch + x;
-        const bool fixed = (nflags[sp.node_off + o] & NF_TYPE) != 0;
-        init_node<S>(fields[k], fields[stride + k], fields[2 * stride + k], fields[3 * stride + k], sp, fr, state, buf2,
-                     buf3, o, fixed);
-    }
+        const int rows = min(IO_Y, sp.ny - y0) * NQ;  // values of a column of the tile
+        Pair<S> v[NQ];
+        if (to_aos && in) {
+#pragma unroll
+            for (int i = 0; i < NQ; ++i) v[i] = pair_base(state, sp)[(long long)i * sp.plane + o];
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            double *a = aos + half * n;
+            auto move = [&](auto one) {
+                for (int k = t; k < IO_X * IO_Y * NQ; k += IO_N) {
+                    const int c = k / (IO_Y * NQ), r = k % (IO_Y * NQ);
+                    if (x0 + c < sp.nx && r < rows) one(a[((long long)(x0 + c) * sp.ny + y0) * NQ + r], buf[c][r]);
+                }
+            };
+            if (to_aos) {
+                if (in) {
+#pragma unroll
+                    for (int i = 0; i < NQ; ++i) buf[lx][ly * NQ + i] = (double)(half ? v[i].y : v[i].x) + fr[half * NQ + i];
+                }
+                __syncthreads();
+                move([](double &g, double &b) { g = b; });
+            } else {
+                move([](double &g, double &b) { b = g; });
+                __syncthreads();
+                if (in) {
+#pragma unroll
+                    for (int i = 0; i < NQ; ++i) {
+                        const S w = (S)(buf[lx][ly * NQ + i] - fr[half * NQ + i]);
+                        if (half) v[i].y = w;
+                        else v[i].x = w;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        if (!to_aos && in) {
+            const bool fixed = (nflags[sp.node_off + o] & NF_TYPE) != 0;  // fixed nodes seed the stage buffers
+#pragma unroll
+            for (int i = 0; i < NQ; ++i) {
+                const long long e = (long long)i * sp.plane + o;
+                pair_base(state, sp)[e] = v[i];
+                if (fixed) {
+                    pair_base(buf2, sp)[e] = v[i];
+                    pair_base(buf3, sp)[e] = v[i];
+                }
+            }
+        }
+    });
+}
+
+// f, h = equilibria of per-node fields (FP64): rho, ux, uy, T, each `stride`
+// values apart
+template <class S>
+__global__ void __launch_bounds__(IO_N) k_set_macro(const SampleParams *samples, int s0, int all, S *state, S *buf2, S *buf3,
+                                                    const double *fields, long long stride, const uint8_t *nflags,
+                                                    const double *fref)
+{
+    __shared__ double buf[4][IO_Y][IO_X + 1];
+    const int s = s0 + blockIdx.y, t = threadIdx.x;
+    const double *fr = fref + NPL * s;
+    const SampleParams &sp = samples[s];
+    if (all) fields += sp.lat_off;
+    io_tiles(sp, [&](int x0, int y0) {
+        {
+            const int lx = t / IO_Y, ly = t % IO_Y, x = x0 + lx, y = y0 + ly;
+            if (x < sp.nx && y < sp.ny) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) buf[k][ly][lx] = fields[k * stride + (long long)x * sp.ny + y];
+            }
+        }
+        __syncthreads();
+        const int lx = t % IO_X, ly = t / IO_X, x = x0 + lx, y = y0 + ly;
+        if (x < sp.nx && y < sp.ny) {
+            const long long o = (long long)y * sp.pitch + x;
+            const bool fixed = (nflags[sp.node_off + o] & NF_TYPE) != 0;
+            init_node<S>(buf[0][ly][lx], buf[1][ly][lx], buf[2][ly][lx], buf[3][ly][lx], sp, fr, state, buf2, buf3, o, fixed);
+        }
+        __syncthreads();
+    });
+}
+
+// blocks for ns samples of up to `nodes` nodes each
+static dim3 io_grid(long long nodes, int ns)
+{
+    const long long tiles = (nodes + IO_N - 1) / IO_N + 1;
+    return dim3((unsigned)std::min<long long>(tiles, ns > 1 ? 256 : 2048), (unsigned)ns);
 }
 
 template <class S>
-cudaError_t launch_set_macro_strided(const SampleParams *samples, int s, S *state, S *buf2, S *buf3,
-                                     const double *fields, long long stride, const uint8_t *nflags, const double *fref,
-                                     long long nodes, cudaStream_t st)
+cudaError_t launch_set_macro(const SampleParams *samples, int s0, int ns, S *state, S *buf2, S *buf3, const double *fields,
+                             long long stride, const uint8_t *nflags, const double *fref, long long nodes, cudaStream_t st)
 {
-    const int blocks = (int)std::min<long long>((nodes + 255) / 256, 4096);
-    k_set_macro<S><<<blocks > 0 ? blocks : 1, 256, 0, st>>>(samples, s, state, buf2, buf3, fields, stride, nflags, fref);
+    k_set_macro<S><<<io_grid(nodes, ns), IO_N, 0, st>>>(samples, s0, ns > 1, state, buf2, buf3, fields, stride, nflags, fref);
     return cudaGetLastError();
 }
-
-template <class S>
-cudaError_t launch_set_macro(const SampleParams *samples, int s, S *state, S *buf2, S *buf3, const double *fields,
-                             const uint8_t *nflags, const double *fref, long long nodes, cudaStream_t st)
-{
-    return launch_set_macro_strided<S>(samples, s, state, buf2, buf3, fields, nodes, nflags, fref, nodes, st);
-}
-template cudaError_t launch_set_macro_strided<double>(const SampleParams *, int, double *, double *, double *,
-                                                      const double *, long long, const uint8_t *, const double *,
-                                                      long long, cudaStream_t);
-template cudaError_t launch_set_macro_strided<float>(const SampleParams *, int, float *, float *, float *,
-                                                     const double *, long long, const uint8_t *, const double *,
-                                                     long long, cudaStream_t);
-template cudaError_t launch_set_macro<double>(const SampleParams *, int, double *, double *, double *, const double *,
-                                              const uint8_t *, const double *, long long, cudaStream_t);
-template cudaError_t launch_set_macro<float>(const SampleParams *, int, float *, float *, float *, const double *,
-                                             const uint8_t *, const double *, long long, cudaStream_t);
+template cudaError_t launch_set_macro<double>(const SampleParams *, int, int, double *, double *, double *, const double *,
+                                              long long, const uint8_t *, const double *, long long, cudaStream_t);
+template cudaError_t launch_set_macro<float>(const SampleParams *, int, int, float *, float *, float *, const double *,
+                                             long long, const uint8_t *, const double *, long long, cudaStream_t);
 
 // ----------------------------------------------------------------- launchers
 // phase: 0 pointwise stages, 1 stencil phase over buffer 2, 2 RK3 final
@@ -322,27 +389,18 @@ cudaError_t launch_init(const KArgs<S> &a, const double *rho, const double *ux, 
 }
 
 template <class S>
-cudaError_t launch_macro_out_strided(const SampleParams *samples, int s, const S *state, double *out,
-                                     long long stride, long long nodes, cudaStream_t st)
+cudaError_t launch_macro_out(const SampleParams *samples, int s0, int ns, const S *state, double *out, long long stride,
+                             long long nodes, cudaStream_t st)
 {
-    const int blocks = (int)std::min<long long>((nodes + 255) / 256, 4096);
-    k_macro_out<S><<<blocks > 0 ? blocks : 1, 256, 0, st>>>(samples, s, state, out, stride);
+    k_macro_out<S><<<io_grid(nodes, ns), IO_N, 0, st>>>(samples, s0, ns > 1, state, out, stride);
     return cudaGetLastError();
-}
-
-template <class S>
-cudaError_t launch_macro_out(const SampleParams *samples, int s, const S *state, double *out, long long nodes,
-                             cudaStream_t st)
-{
-    return launch_macro_out_strided<S>(samples, s, state, out, nodes, nodes, st);
 }
 
 template <class S>
 cudaError_t launch_dist_io(const SampleParams *samples, int s, S *state, S *buf2, S *buf3, double *aos, int to_aos,
                            const uint8_t *nflags, const double *fref, long long nodes, cudaStream_t st)
 {
-    const int blocks = (int)std::min<long long>((nodes * NQ + 255) / 256, 8192);
-    k_dist_io<S><<<blocks > 0 ? blocks : 1, 256, 0, st>>>(samples, s, state, buf2, buf3, aos, to_aos, nflags, fref);
+    k_dist_io<S><<<io_grid(nodes, 1), IO_N, 0, st>>>(samples, s, state, buf2, buf3, aos, to_aos, nflags, fref);
     return cudaGetLastError();
 }
 
@@ -388,12 +446,10 @@ template cudaError_t launch_init<double>(const KArgs<double> &, const double *, 
                                          const double *, cudaStream_t);
 template cudaError_t launch_init<float>(const KArgs<float> &, const double *, const double *, const double *,
                                         const double *, cudaStream_t);
-template cudaError_t launch_macro_out_strided<double>(const SampleParams *, int, const double *, double *, long long,
-                                                      long long, cudaStream_t);
-template cudaError_t launch_macro_out_strided<float>(const SampleParams *, int, const float *, double *, long long,
-                                                     long long, cudaStream_t);
-template cudaError_t launch_macro_out<double>(const SampleParams *, int, const double *, double *, long long, cudaStream_t);
-template cudaError_t launch_macro_out<float>(const SampleParams *, int, const float *, double *, long long, cudaStream_t);
+template cudaError_t launch_macro_out<double>(const SampleParams *, int, int, const double *, double *, long long, long long,
+                                              cudaStream_t);
+template cudaError_t launch_macro_out<float>(const SampleParams *, int, int, const float *, double *, long long, long long,
+                                             cudaStream_t);
 template cudaError_t launch_dist_io<double>(const SampleParams *, int, double *, double *, double *, double *, int,
                                             const uint8_t *, const double *, long long, cudaStream_t);
 template cudaError_t launch_dist_io<float>(const SampleParams *, int, float *, float *, float *, double *, int,

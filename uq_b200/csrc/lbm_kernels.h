@@ -78,24 +78,18 @@ cudaError_t prepare_flux();
 template <class S>
 cudaError_t launch_init(const KArgs<S> &a, const double *rho, const double *ux, const double *uy, const double *T,
                         cudaStream_t st);
+// boundary I/O of samples s0 .. s0 + ns - 1, `nodes` the most nodes of one;
+// fields `stride` values apart, of one sample, or (ns > 1) of every sample
+// SampleParams::lat_off values in
 template <class S>
-cudaError_t launch_macro_out(const SampleParams *samples, int s, const S *state, double *out, long long nodes,
-                             cudaStream_t st);
-// the same with the fields `stride` values apart (several samples' fields
-// in one buffer)
+cudaError_t launch_macro_out(const SampleParams *samples, int s0, int ns, const S *state, double *out, long long stride,
+                             long long nodes, cudaStream_t st);
 template <class S>
-cudaError_t launch_macro_out_strided(const SampleParams *samples, int s, const S *state, double *out,
-                                     long long stride, long long nodes, cudaStream_t st);
-template <class S>
-cudaError_t launch_set_macro_strided(const SampleParams *samples, int s, S *state, S *buf2, S *buf3,
-                                     const double *fields, long long stride, const uint8_t *nflags, const double *fref,
-                                     long long nodes, cudaStream_t st);
+cudaError_t launch_set_macro(const SampleParams *samples, int s0, int ns, S *state, S *buf2, S *buf3, const double *fields,
+                             long long stride, const uint8_t *nflags, const double *fref, long long nodes, cudaStream_t st);
 template <class S>
 cudaError_t launch_dist_io(const SampleParams *samples, int s, S *state, S *buf2, S *buf3, double *aos, int to_aos,
                            const uint8_t *nflags, const double *fref, long long nodes, cudaStream_t st);
-template <class S>
-cudaError_t launch_set_macro(const SampleParams *samples, int s, S *state, S *buf2, S *buf3, const double *fields,
-                             const uint8_t *nflags, const double *fref, long long nodes, cudaStream_t st);
 cudaError_t launch_wait_selftest(int *status, int arrive, cudaStream_t st);
 // copy the edge columns of stage buffers 2 and 3 into the ghost columns
 // (SampleParams::gx) of samples s0 .. s0 + ns - 1 (after their state was set)

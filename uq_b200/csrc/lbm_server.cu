@@ -597,11 +597,11 @@ struct lbm_server {
         }
         CU(cudaMemcpyAsync(scratch.p, r->fields.data(), sizeof(double) * 4 * n, cudaMemcpyHostToDevice, stream));
         if (prec == LBM_PREC_F64)
-            CU(launch_set_macro<double>(d_sp.p, k, reinterpret_cast<double *>(state.p), reinterpret_cast<double *>(buf2.p),
-                                        reinterpret_cast<double *>(buf3.p), scratch.p, nflags.p, d_fref.p, n, stream));
+            CU(launch_set_macro<double>(d_sp.p, k, 1, reinterpret_cast<double *>(state.p), reinterpret_cast<double *>(buf2.p),
+                                        reinterpret_cast<double *>(buf3.p), scratch.p, n, nflags.p, d_fref.p, n, stream));
         else
-            CU(launch_set_macro<float>(d_sp.p, k, reinterpret_cast<float *>(state.p), reinterpret_cast<float *>(buf2.p),
-                                       reinterpret_cast<float *>(buf3.p), scratch.p, nflags.p, d_fref.p, n, stream));
+            CU(launch_set_macro<float>(d_sp.p, k, 1, reinterpret_cast<float *>(state.p), reinterpret_cast<float *>(buf2.p),
+                                       reinterpret_cast<float *>(buf3.p), scratch.p, n, nflags.p, d_fref.p, n, stream));
         // the ghost columns of the new solve's stage buffers (SampleParams::gx)
         if (r->ps.p.gx) {
             if (prec == LBM_PREC_F64)
@@ -791,9 +791,9 @@ struct lbm_server {
             while (packed[k] != r) ++k;
             const long long n = (long long)r->nx * r->ny;
             if (prec == LBM_PREC_F64)
-                CU(launch_macro_out<double>(d_sp.p, (int)k, reinterpret_cast<double *>(state.p), result_ptr(r), n, stream));
+                CU(launch_macro_out<double>(d_sp.p, (int)k, 1, reinterpret_cast<double *>(state.p), result_ptr(r), n, n, stream));
             else
-                CU(launch_macro_out<float>(d_sp.p, (int)k, reinterpret_cast<float *>(state.p), result_ptr(r), n, stream));
+                CU(launch_macro_out<float>(d_sp.p, (int)k, 1, reinterpret_cast<float *>(state.p), result_ptr(r), n, n, stream));
         }
         std::shared_ptr<Snapshot> snap = enqueue_snapshot();
         {
