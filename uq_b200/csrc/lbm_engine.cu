@@ -461,9 +461,23 @@ struct lbm_batch {
     DevBuf<WallNode> d_walls_all, d_walls_rk3, d_every_wall, d_every_wall_rk3;
     DevBuf<CUtensorMap> d_maps;
     DevBuf<double> d_fref;
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // [want_residual]
+    // one step with and without the residual, and kGraphSteps steps: a graph's
+    // own launch costs a small solve as much as one of its kernels
+    static constexpr int kGraphSteps = 8;
+    cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};  // [want_residual], several steps
     std::vector<int> host_status;
     std::vector<double> host_residual;
+    // pinned: n residuals, then n status words
+    struct Report {
+        double *p = nullptr;
+        void alloc(size_t n) { CU(cudaHostAlloc(&p, n * (sizeof(double) + sizeof(int)), cudaHostAllocDefault)); }
+        double *residual() const { return p; }
+        int *status(size_t n) const { return reinterpret_cast<int *>(p + n); }
+        ~Report()
+        {
+            if (p) cudaFreeHost(p);
+        }
+    } report;
 
     size_t elem() const { return prec == LBM_PREC_F64 ? 8 : 4; }
 
@@ -699,6 +713,7 @@ struct lbm_batch {
         scratch.alloc(std::max<size_t>(5 * max_nodes, 2 * 13 * max_nodes));
         host_status.assign(n, 0);
         host_residual.assign(n, 1.0);
+        report.alloc(n);
 
         make_maps();
         if (prec == LBM_PREC_F64) CU((prepare_kernels<double, double>()));
@@ -875,42 +890,52 @@ struct lbm_batch {
 
     void launch_steps(int n, int want_res)
     {
-        const int g = want_res ? 1 : 0;
-        if (use_graph && !graph[g]) {
-            cudaGraph_t gr;
-            CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-            try {
-                enqueue_step(want_res);
-            } catch (...) {
-                cudaStreamEndCapture(stream, &gr);
-                throw;
-            }
-            CU(cudaStreamEndCapture(stream, &gr));
-            CU(cudaGraphInstantiate(&graph[g], gr, 0));
-            cudaGraphDestroy(gr);
+        if (!use_graph) {
+            for (int k = 0; k < n; ++k) enqueue_step(want_res);
+            return;
         }
-        for (int k = 0; k < n; ++k) {
-            if (use_graph) CU(cudaGraphLaunch(graph[g], stream));
-            else enqueue_step(want_res);
-        }
+        if (!want_res)
+            for (; n >= kGraphSteps; n -= kGraphSteps) CU(cudaGraphLaunch(step_graph(2), stream));
+        for (; n > 0; --n) CU(cudaGraphLaunch(step_graph(want_res ? 1 : 0), stream));
     }
 
-    // collect and clear the per-sample status words
-    void fetch_status()
+    cudaGraphExec_t step_graph(int g)
     {
-        std::vector<int> st(hs.size());
-        CU(cudaMemcpyAsync(st.data(), status.p, st.size() * sizeof(int), cudaMemcpyDeviceToHost, stream));
-        CU(cudaMemsetAsync(status.p, 0, st.size() * sizeof(int), stream));
-        CU(cudaStreamSynchronize(stream));
-        for (size_t k = 0; k < st.size(); ++k) host_status[k] |= st[k];
+        if (graph[g]) return graph[g];
+        cudaGraph_t gr;
+        CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        try {
+            for (int k = 0; k < (g == 2 ? kGraphSteps : 1); ++k) enqueue_step(g == 1);
+        } catch (...) {
+            cudaStreamEndCapture(stream, &gr);
+            throw;
+        }
+        CU(cudaStreamEndCapture(stream, &gr));
+        const cudaError_t e = cudaGraphInstantiate(&graph[g], gr, 0);
+        cudaGraphDestroy(gr);
+        CU(e);
+        return graph[g];
     }
 
-    void fetch_residual()
+    // What a step reports, read back into pinned memory with one
+    // synchronisation: the per-sample status words (collected and cleared) and,
+    // when asked for, the residuals.
+    void fetch(bool with_status, bool with_residual)
     {
-        CU(cudaMemcpyAsync(host_residual.data(), residual.p, host_residual.size() * sizeof(double),
-                           cudaMemcpyDeviceToHost, stream));
+        const size_t n = hs.size();
+        if (with_residual)
+            CU(cudaMemcpyAsync(report.residual(), residual.p, n * sizeof(double), cudaMemcpyDeviceToHost, stream));
+        if (with_status) {
+            CU(cudaMemcpyAsync(report.status(n), status.p, n * sizeof(int), cudaMemcpyDeviceToHost, stream));
+            CU(cudaMemsetAsync(status.p, 0, n * sizeof(int), stream));
+        }
         CU(cudaStreamSynchronize(stream));
+        if (with_residual) std::copy(report.residual(), report.residual() + n, host_residual.begin());
+        if (with_status)
+            for (size_t k = 0; k < n; ++k) host_status[k] |= report.status(n)[k];
     }
+    void fetch_status() { fetch(true, false); }
+    void fetch_residual() { fetch(false, true); }
 
     static lbm_status to_status(int bits)
     {
@@ -1096,18 +1121,14 @@ lbm_status lbm_step(lbm_handle *h, int n_steps, int want_residual, double *resid
     HostSample &s = b.hs[0];
     b.host_status[0] = 0;
     if (want_residual) {
-        // the residual belongs to each step; step one at a time
-        for (int k = 0; k < n_steps; ++k) {
-            s.step += 1;
-            b.launch_steps(1, 1);
-            b.fetch_residual();
-            s.residual = b.host_residual[0];
-        }
+        // the residual is that of the last step
+        b.launch_steps(n_steps, 1);
     } else {
         b.launch_steps(n_steps, 0);
-        s.step += n_steps;
     }
-    b.fetch_status();
+    s.step += n_steps;
+    b.fetch(true, want_residual && n_steps > 0);
+    if (want_residual && n_steps > 0) s.residual = b.host_residual[0];
     if (residual_out) *residual_out = s.residual;
     return lbm_batch::to_status(b.host_status[0]);
     API_END
@@ -1127,8 +1148,7 @@ lbm_status lbm_run(lbm_handle *h, int max_steps, int *stop_out, double *trace, i
         b.host_status[0] = 0;
         if (s.tol != 0) {
             b.launch_steps(1, 1);
-            b.fetch_residual();
-            b.fetch_status();
+            b.fetch(true, true);
             s.residual = b.host_residual[0];
             stop = (b.host_status[0] & STATUS_EQ) ? 1 : 0;
             if (s.step >= 2 && s.step <= numRes) {

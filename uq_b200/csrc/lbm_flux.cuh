@@ -504,6 +504,7 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
         if (active) load();
         __syncthreads();
     }
+    pdl_trigger();
     double res_part = 0;
     if (active) {
         const S *stage = MODE == 2 ? a.buf3 : a.buf2;
@@ -736,6 +737,7 @@ __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP &&
             mbar_init(&bars[ix - 1], 1);
             if (warp < 4) mbar_init(&bars[ix], 1);
             fence_mbar_init();
+            pdl_wait();
             issue_warp<S>(t, maps, sm, bars, warp);
         }
     } else if constexpr (SWEEP) {
@@ -750,6 +752,7 @@ __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP &&
             reinterpret_cast<int *>(&s_sp)[k] = reinterpret_cast<const int *>(gsp)[k];
         if (tid == 0) s_tile = t;
     }
+    pdl_wait();
     // (what a plain tile's sweeps need is in the tile itself)
     if (!TC || !SWEEP || flux_early<S>(MODE) || (t.kind & TILE_FIX)) __syncthreads();
     const SampleParams &sp = s_sp;
@@ -838,13 +841,15 @@ cudaError_t launch_flux(int mode, const KArgs<S> &a, int ntiles, int path, cudaS
     k.slots = def ? 12 : flux_slots<S>(k.tx, k.ty);
     const int NT = k.tx * k.ty;
     const size_t sm = flux_smem_bytes_t<S>(k.tx, k.ty, sweep);
+    cudaError_t e = cudaSuccess;
     with_mode(mode, [&](auto m) {
         constexpr int M = decltype(m)::value;
-        if (!sweep) k_flux<S, M, FLUX_GENERAL, false><<<ntiles, NT, sm, st>>>(k);
-        else if (!def) k_flux<S, M, FLUX_SWEEP, false><<<ntiles, NT, sm, st>>>(k);
-        else k_flux<S, M, FLUX_SWEEP, true><<<ntiles, NT, sm, st>>>(k);
+        e = launch_step_kernel(!sweep ? k_flux<S, M, FLUX_GENERAL, false>
+                               : def  ? k_flux<S, M, FLUX_SWEEP, true>
+                                      : k_flux<S, M, FLUX_SWEEP, false>,
+                               ntiles, NT, sm, st, !k.phased, k);
     });
-    return cudaGetLastError();
+    return e;
 }
 
 template <class S>

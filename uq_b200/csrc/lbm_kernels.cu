@@ -86,7 +86,9 @@ __global__ void __launch_bounds__(256, Stage0Blocks<S>::value) k_stage0(KArgs<S>
     if (x >= sp.nx || y >= sp.ny) return;
     const int o = y * sp.pitch + x, PL = (int)sp.plane;
     const long long node = sp.node_off + o;
-    if ((a.nflags[node] & NF_TYPE) != 0) return;
+    const int type = a.nflags[node] & NF_TYPE;
+    pdl_wait();
+    if (type != 0) return;
     const V *__restrict__ st = pair_base(a.state, sp) + o;
     V *__restrict__ b2 = pair_base(a.buf2, sp) + o;
     const int gd = a.phased ? 0 : ghost_offset(sp, x);
@@ -103,6 +105,7 @@ __global__ void __launch_bounds__(256, Stage0Blocks<S>::value) k_stage0(KArgs<S>
         return;
     }
     const Macro m = node_macro_rd([&](int i) { return v[i]; }, sp);
+    pdl_trigger();
     if (a.want_residual) a.told[node] = m.T;
     constexpr bool DEV = sizeof(S) == 4;
     const EqArgs<C, DEV> q(m.rho, m.ux, m.uy, m.T, sp);
@@ -176,15 +179,25 @@ cudaError_t launch_fill_ghosts(const SampleParams *samples, int s0, int ns, S *b
 template cudaError_t launch_fill_ghosts<double>(const SampleParams *, int, int, double *, double *, cudaStream_t);
 template cudaError_t launch_fill_ghosts<float>(const SampleParams *, int, int, float *, float *, cudaStream_t);
 
-// per-sample residual = sqrt(sum / (Nx Ny)) (runOne, cpuLBM.cpp:2322-2331)
-__global__ void k_residual(const SampleParams *samples, int nsamples, const double *partial, const int *tile_first,
-                           const int *tile_count, double *residual)
+// per-sample residual = sqrt(sum / (Nx Ny)) (runOne, cpuLBM.cpp:2322-2331):
+// block s adds sample s's per-tile sums, thread t every 256th, then the
+// threads pairwise (always the same order).  One thread per sample took
+// 0.62 ms over the 16,384 tiles of a 2048 x 2048 grid, more than the step.
+__global__ void __launch_bounds__(256) k_residual(const SampleParams *samples, const double *partial, const int *tile_first,
+                                                  const int *tile_count, double *residual)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nsamples) return;
-    double sum = 0;
-    for (int k = 0; k < tile_count[s]; ++k) sum += partial[tile_first[s] + k];
-    residual[s] = sqrt(sum / ((double)samples[s].nx * samples[s].ny));
+    __shared__ double sum[256];
+    const int s = blockIdx.x, t = threadIdx.x, n = tile_count[s];
+    const double *p = partial + tile_first[s];
+    double v = 0;
+    for (int k = t; k < n; k += 256) v += p[k];
+    sum[t] = v;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if (t < w) sum[t] += sum[t + w];
+        __syncthreads();
+    }
+    if (t == 0) residual[s] = sqrt(sum[0] / ((double)samples[s].nx * samples[s].ny));
 }
 
 // ------------------------------------------------------------ boundary I/O
@@ -361,9 +374,8 @@ cudaError_t launch_phase(const KArgs<S> &a, int phase, int rk, const Tile *tiles
     const int NT = a.tx * a.ty;
     if (phase == 0) {
         if (!ntiles) return cudaSuccess;
-        if (rk == 1) k_stage0<S, 1><<<ntiles, NT, 0, st>>>(k);
-        else if (rk == 0) k_stage0<S, 0><<<ntiles, NT, 0, st>>>(k);
-        else k_stage0<S, 2><<<ntiles, NT, 0, st>>>(k);
+        return launch_step_kernel(rk == 1 ? k_stage0<S, 1> : rk == 0 ? k_stage0<S, 0> : k_stage0<S, 2>, ntiles, NT, 0, st,
+                                  !k.phased, k);
     } else if (phase == 1 || phase == 2) {
         if (!ntiles) return cudaSuccess;
         const int mode = phase == 2 ? 2 : (rk == 1 ? 1 : (rk == 0 ? 3 : (rk == 2 ? 4 : 5)));
@@ -432,7 +444,7 @@ cudaError_t launch_wait_selftest(int *status, int arrive, cudaStream_t st)
 cudaError_t launch_residual(const SampleParams *samples, int nsamples, const double *partial, const int *tile_first,
                             const int *tile_count, double *residual, cudaStream_t st)
 {
-    k_residual<<<(nsamples + 127) / 128, 128, 0, st>>>(samples, nsamples, partial, tile_first, tile_count, residual);
+    k_residual<<<nsamples, 256, 0, st>>>(samples, partial, tile_first, tile_count, residual);
     return cudaGetLastError();
 }
 

@@ -61,6 +61,33 @@ struct KArgs {
 #endif
 };
 
+// Programmatic dependent launch: a kernel of a step starts while the one
+// before it drains, and waits (pdl_wait) before it touches what that one
+// writes; until then it reads only what no step changes (tiles, sample
+// parameters, node flags).  A launch gap and a block's first look-ups are
+// most of a small solve's kernel.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_step_kernel(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, bool overlap,
+                               A... args)
+{
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+#endif
+
 // Which tiles a stencil-phase launch covers: the sweep tiles or the general
 // tiles of its list, one kernel each (see TILE_SWEEP).
 enum FluxPath { FLUX_SWEEP = 1, FLUX_GENERAL = 2 };
