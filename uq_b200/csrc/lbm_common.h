@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 namespace uqlbm {
@@ -69,7 +70,9 @@ struct HostSample {
     int nsteps = 0;
     std::vector<double> dx, dy;
     std::vector<uint8_t> type;  // [y*nx + x]
-    std::vector<double> rho0, ux0, uy0, T0;  // [y*nx + x] initial node state
+    // initial node state rho, ux, uy, T, each nx ny values in the boundary's
+    // [x*ny + y] order (freed once on the device)
+    std::unique_ptr<double[]> fields;
     // driver state (cpuLBM::step, residual, initRes, resNorm; main.cpp:34-70)
     int step = 0;
     double residual = 1, resNorm = 0, initRes[100] = {0};

@@ -173,21 +173,22 @@ HostSample derive(const lbm_config &c, const lbm_init &in)
     }
     const size_t N = (size_t)Nx * Ny;
     s.type.resize(N);
-    s.rho0.resize(N);
-    s.ux0.resize(N);
-    s.uy0.resize(N);
-    s.T0.resize(N);
-    for (int x = 0; x < Nx; ++x)
-        for (int y = 0; y < Ny; ++y) {
-            const int id = in.bndArray[(size_t)x * Ny + y];
-            if (id < 0 || id >= np) throw LbmError(LBM_ERR_INVALID, "bndArray holds an unknown property id");
-            const size_t k = (size_t)y * Nx + x;
-            s.type[k] = (uint8_t)in.cellType[id];
-            s.rho0[k] = prho[id];
-            s.ux0[k] = in.velocityX[id];
-            s.uy0[k] = in.velocityY[id];
-            s.T0[k] = pT[id];
-        }
+    s.fields.reset(new double[4 * N]);
+    double *rho0 = s.fields.get(), *ux0 = rho0 + N, *uy0 = ux0 + N, *T0 = uy0 + N;
+    for (size_t k = 0; k < N; ++k) {
+        const int id = in.bndArray[k];
+        if (id < 0 || id >= np) throw LbmError(LBM_ERR_INVALID, "bndArray holds an unknown property id");
+        rho0[k] = prho[id];
+        ux0[k] = in.velocityX[id];
+        uy0[k] = in.velocityY[id];
+        T0[k] = pT[id];
+    }
+    // the cell types with x fastest, 64 x 64 nodes at a time
+    for (int xb = 0; xb < Nx; xb += 64)
+        for (int yb = 0; yb < Ny; yb += 64)
+            for (int y = yb; y < std::min(yb + 64, Ny); ++y)
+                for (int x = xb; x < std::min(xb + 64, Nx); ++x)
+                    s.type[(size_t)y * Nx + x] = (uint8_t)in.cellType[in.bndArray[(size_t)x * Ny + y]];
     return s;
 }
 
@@ -253,7 +254,7 @@ void prepare_sample(const HostSample &h, int prec, PreparedSample &out)
         // is moderate.  Bound those values by the initial densities and the
         // energy scale rho R Tc (times generous factors for the polynomials).
         double rho_max = 0.0;
-        for (double r : h.rho0) rho_max = std::max(rho_max, std::fabs(r));
+        for (size_t k = 0; k < (size_t)h.nx * h.ny; ++k) rho_max = std::max(rho_max, std::fabs(h.fields[k]));
         const double scale = 2.0 * h.c * rho_max * std::max(2.0, 10.0 * h.R * h.Tc);
         p.wide = (prec == LBM_PREC_F32 && !(scale <= 100.0)) ? 1 : 0;
         // the FP64 reconstructions' epsilon, kept where its powers are normal
@@ -297,26 +298,45 @@ void prepare_sample(const HostSample &h, int prec, PreparedSample &out)
     out.dy.resize(h.ny);
     for (int x = 0; x < h.nx; ++x) { out.tdx[x] = h.dt / h.dx[x]; out.dx[x] = h.dx[x]; }
     for (int y = 0; y < h.ny; ++y) { out.tdy[y] = h.dt / h.dy[y]; out.dy[y] = h.dy[y]; }
-    // node flags
+    // node flags: the cell type, solids within two nodes along each axis, and
+    // the two nodes at each edge.  Only rows with a solid in them, and the two
+    // on either side of those, are looked at node by node.
     out.flags.assign((size_t)p.plane, 0);
+    std::vector<uint8_t> has_solid(h.ny, 0);
     int m;
-    for (int y = 0; y < h.ny; ++y)
+    for (int y = 0; y < h.ny; ++y) {
+        const uint8_t *type = &h.type[(size_t)y * h.nx];
+        uint8_t *fl = &out.flags[(size_t)y * p.pitch], any = 0;
+        const uint8_t edge = y < 2 || y > h.ny - 3 ? ((h.flags & SF_PERY) ? NF_WRPY : NF_EDGY) : 0;
         for (int x = 0; x < h.nx; ++x) {
-            uint8_t fl = h.type[(size_t)y * h.nx + x];
-            for (int d = -2; d <= 2; ++d) {
-                const int xr = host_bc_index(h, x, d, 0, m);
-                const int yr = host_bc_index(h, y, d, 1, m);
-                if (h.type[(size_t)y * h.nx + xr] == 2) fl |= NF_SOLX;
-                if (h.type[(size_t)yr * h.nx + x] == 2) fl |= NF_SOLY;
-            }
-            if (x < 2 || x > h.nx - 3) fl |= (h.flags & SF_PERX) ? NF_WRPX : NF_EDGX;
-            if (y < 2 || y > h.ny - 3) fl |= (h.flags & SF_PERY) ? NF_WRPY : NF_EDGY;
-            out.flags[(size_t)y * p.pitch + x] = fl;
+            fl[x] = type[x] | edge;
+            any |= type[x] == 2;
         }
+        for (int x = 0; x < h.nx; ++x) {
+            if (x == 2) x = std::max(2, h.nx - 2);  // the two columns at each edge
+            if (x < h.nx) fl[x] |= (h.flags & SF_PERX) ? NF_WRPX : NF_EDGX;
+        }
+        has_solid[y] = any;
+    }
+    for (int y = 0; y < h.ny; ++y) {
+        uint8_t *fl = &out.flags[(size_t)y * p.pitch];
+        if (has_solid[y])
+            for (int x = 0; x < h.nx; ++x)
+                for (int d = -2; d <= 2; ++d)
+                    if (h.type[(size_t)y * h.nx + host_bc_index(h, x, d, 0, m)] == 2) fl[x] |= NF_SOLX;
+        for (int d = -2; d <= 2; ++d) {
+            const int yr = host_bc_index(h, y, d, 1, m);
+            if (!has_solid[yr]) continue;
+            const uint8_t *type = &h.type[(size_t)yr * h.nx];
+            for (int x = 0; x < h.nx; ++x)
+                if (type[x] == 2) fl[x] |= NF_SOLY;
+        }
+    }
     // wall nodes: solid with a non-solid 4-neighbour (wallFluxes' test)
     static const int wx[4] = {-1, 1, 0, 0}, wy[4] = {0, 0, -1, 1};
     out.walls.clear();
-    for (int y = 0; y < h.ny; ++y)
+    for (int y = 0; y < h.ny; ++y) {
+        if (!has_solid[y]) continue;
         for (int x = 0; x < h.nx; ++x) {
             if (h.type[(size_t)y * h.nx + x] != 2) continue;
             bool adj = false;
@@ -327,6 +347,7 @@ void prepare_sample(const HostSample &h, int prec, PreparedSample &out)
             }
             if (adj) out.walls.push_back(WallNode{0, x, y, 0});
         }
+    }
 }
 
 // Tiles of one sample with their kinds.  A tile is a sweep tile when all
@@ -719,31 +740,18 @@ struct lbm_batch {
         if (prec == LBM_PREC_F64) CU((prepare_kernels<double, double>()));
         else CU((prepare_kernels<float, float>()));
 
-        // initial state (initialiseFunctions, cpuLBM.cpp:846-875)
-        std::vector<double> r0(total_nodes, 1.0), u0(total_nodes, 0.0), v0(total_nodes, 0.0), T0(total_nodes, 1.0);
-        for (int k = 0; k < n; ++k) {
-            const HostSample &h = hs[k];
-            for (int y = 0; y < h.ny; ++y)
-                for (int x = 0; x < h.nx; ++x) {
-                    const size_t src = (size_t)y * h.nx + x;
-                    const long long dst = sp[k].node_off + (long long)y * sp[k].pitch + x;
-                    r0[dst] = h.rho0[src];
-                    u0[dst] = h.ux0[src];
-                    v0[dst] = h.uy0[src];
-                    T0[dst] = h.T0[src];
-                }
-        }
-        DevBuf<double> dr, du, dv, dT;
-        dr.upload(r0, stream);
-        du.upload(u0, stream);
-        dv.upload(v0, stream);
-        dT.upload(T0, stream);
-        if (prec == LBM_PREC_F64) CU(launch_init<double>(args<double>(0), dr.p, du.p, dv.p, dT.p, stream));
-        else CU(launch_init<float>(args<float>(0), dr.p, du.p, dv.p, dT.p, stream));
-        fill_ghosts(0, n);
+        // initial state (initialiseFunctions, cpuLBM.cpp:846-875), by the
+        // kernel that sets a state from fields
+        DevBuf<double> init;
+        init.alloc(4 * lattice_nodes);
+        for (int k = 0; k < n; ++k)
+            CU(cudaMemcpyAsync(init.p + 4 * sp[k].lat_off, hs[k].fields.get(),
+                               sizeof(double) * 4 * hs[k].nx * (size_t)hs[k].ny, cudaMemcpyHostToDevice, stream));
+        write_fields(0, n, init.p, 0, (long long)max_nodes);
         CU(cudaStreamSynchronize(stream));
         // equilibrium failures during initialisation are not reported by the
         // reference (hasFailed is reset by runOne, cpuLBM.cpp:2288)
+        for (HostSample &h : hs) h.fields.reset();
         CU(cudaMemsetAsync(status.p, 0, n * sizeof(int), stream));
         CU(cudaStreamSynchronize(stream));
     }
@@ -829,7 +837,8 @@ struct lbm_batch {
     }
 
     // the state of samples s0 .. s0 + ns - 1 from fields on the device,
-    // `stride` values apart (`nodes`: the most nodes of one)
+    // `stride` values apart, or (0) sample by sample, each one's four fields
+    // together (`nodes`: the most nodes of one)
     void write_fields(int s0, int ns, const double *fields, long long stride, long long nodes)
     {
         if (prec == LBM_PREC_F64)

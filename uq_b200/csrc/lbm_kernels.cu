@@ -49,22 +49,6 @@ __device__ __noinline__ bool init_node(double rho, double ux, double uy, double 
     return !(fabs(sf - rho) > 1e-6);
 }
 
-template <class S>
-__global__ void k_init(KArgs<S> a, const double *__restrict__ rho, const double *__restrict__ ux,
-                       const double *__restrict__ uy, const double *__restrict__ T)
-{
-    const Tile t = a.tiles[blockIdx.x];
-    const SampleParams sp = a.samples[t.sample];
-    const int x = t.x0 + threadIdx.x % a.tx, y = t.y0 + threadIdx.x / a.tx;
-    if (x >= sp.nx || y >= sp.ny) return;
-    const long long node = sp.node_off + (long long)y * sp.pitch + x;
-    const bool fixed = (a.nflags[node] & NF_TYPE) != 0;
-    const long long o = (long long)y * sp.pitch + x;
-    if (!init_node<S>(rho[node], ux[node], uy[node], T[node], sp, a.fref + NPL * t.sample, a.state, a.buf2, a.buf3, o,
-                      fixed))
-        atomicOr(&a.status[t.sample], STATUS_EQ);
-}
-
 // ------------------------------------------------------------------- P0
 // RK: 1 (RK3 stages 1+2), 0 (RK1 stage 1), 2 (EULER / EULER_EQ: copy).
 // Pointwise and memory-bound.  A node's 13 pairs are loaded once and stay in
@@ -322,6 +306,10 @@ __global__ void __launch_bounds__(IO_N) k_set_macro(const SampleParams *samples,
     const double *fr = fref + NPL * s;
     const SampleParams &sp = samples[s];
     if (all) fields += sp.lat_off;
+    if (!stride) {  // the samples' four fields together
+        fields += 4 * sp.lat_off - (all ? sp.lat_off : 0);
+        stride = (long long)sp.nx * sp.ny;
+    }
     io_tiles(sp, [&](int x0, int y0) {
         {
             const int lx = t / IO_Y, ly = t % IO_Y, x = x0 + lx, y = y0 + ly;
@@ -393,14 +381,6 @@ cudaError_t prepare_kernels()
 }
 
 template <class S>
-cudaError_t launch_init(const KArgs<S> &a, const double *rho, const double *ux, const double *uy, const double *T,
-                        cudaStream_t st)
-{
-    if (a.ntiles) k_init<S><<<a.ntiles, a.tx * a.ty, 0, st>>>(a, rho, ux, uy, T);
-    return cudaGetLastError();
-}
-
-template <class S>
 cudaError_t launch_macro_out(const SampleParams *samples, int s0, int ns, const S *state, double *out, long long stride,
                              long long nodes, cudaStream_t st)
 {
@@ -454,10 +434,6 @@ template cudaError_t launch_phase<float, float>(const KArgs<float> &, int, int, 
                                                 cudaStream_t, int);
 template cudaError_t prepare_kernels<double, double>();
 template cudaError_t prepare_kernels<float, float>();
-template cudaError_t launch_init<double>(const KArgs<double> &, const double *, const double *, const double *,
-                                         const double *, cudaStream_t);
-template cudaError_t launch_init<float>(const KArgs<float> &, const double *, const double *, const double *,
-                                        const double *, cudaStream_t);
 template cudaError_t launch_macro_out<double>(const SampleParams *, int, int, const double *, double *, long long, long long,
                                               cudaStream_t);
 template cudaError_t launch_macro_out<float>(const SampleParams *, int, int, const float *, double *, long long, long long,

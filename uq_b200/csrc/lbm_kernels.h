@@ -102,12 +102,10 @@ template <class S>
 cudaError_t launch_flux(int mode, const KArgs<S> &a, int ntiles, int path, cudaStream_t st);
 template <class S>
 cudaError_t prepare_flux();
-template <class S>
-cudaError_t launch_init(const KArgs<S> &a, const double *rho, const double *ux, const double *uy, const double *T,
-                        cudaStream_t st);
 // boundary I/O of samples s0 .. s0 + ns - 1, `nodes` the most nodes of one;
 // fields `stride` values apart, of one sample, or (ns > 1) of every sample
-// SampleParams::lat_off values in
+// SampleParams::lat_off values in (set: stride 0, each sample's four fields
+// together, 4 lat_off values in)
 template <class S>
 cudaError_t launch_macro_out(const SampleParams *samples, int s0, int ns, const S *state, double *out, long long stride,
                              long long nodes, cudaStream_t st);

@@ -48,7 +48,7 @@ struct Request {
     PreparedSample ps;
     std::vector<Tile> tiles;     // local: sample 0, gid = local index
     std::vector<WallNode> walls; // wall nodes that its general tiles need
-    std::vector<double> fields;  // rho, ux, uy, T in [x*Ny + y] order until admitted
+    std::unique_ptr<double[]> fields;  // rho, ux, uy, T in [x*Ny + y] order until admitted
     std::vector<double> result;  // rho, ux, uy, T, p in [x*Ny + y] order when done
     long long nodes = 0;         // arena slots
     long long node_off = -1;
@@ -287,17 +287,7 @@ struct lbm_server {
         r->nodes = r->ps.p.plane + (r->ps.p.gx ? (GHOST_SLACK + NPL - 1) / NPL : 0);
         cut_tiles(r->ps.flags.data(), r->ps.p, tx, ty, 0, r->tiles);
         needed_walls(r->ps.p, tx, ty, r->tiles.data(), r->ps.walls, r->walls);
-        const long long n = (long long)h.nx * h.ny;
-        r->fields.resize(4 * n);
-        for (int x = 0; x < h.nx; ++x)
-            for (int y = 0; y < h.ny; ++y) {
-                const size_t src = (size_t)y * h.nx + x;
-                const long long k = (long long)x * h.ny + y;
-                r->fields[k] = h.rho0[src];
-                r->fields[n + k] = h.ux0[src];
-                r->fields[2 * n + k] = h.uy0[src];
-                r->fields[3 * n + k] = h.T0[src];
-            }
+        r->fields = std::move(h.fields);
         std::lock_guard<std::mutex> g(mu);
         if (fatal != LBM_OK) throw LbmError(fatal, fatal_msg);
         if (stopping) throw LbmError(LBM_ERR_INVALID, "server is stopping");
@@ -595,7 +585,7 @@ struct lbm_server {
             CU(cudaStreamSynchronize(stream));
             scratch.alloc((size_t)4 * n);
         }
-        CU(cudaMemcpyAsync(scratch.p, r->fields.data(), sizeof(double) * 4 * n, cudaMemcpyHostToDevice, stream));
+        CU(cudaMemcpyAsync(scratch.p, r->fields.get(), sizeof(double) * 4 * n, cudaMemcpyHostToDevice, stream));
         if (prec == LBM_PREC_F64)
             CU(launch_set_macro<double>(d_sp.p, k, 1, reinterpret_cast<double *>(state.p), reinterpret_cast<double *>(buf2.p),
                                         reinterpret_cast<double *>(buf3.p), scratch.p, n, nflags.p, d_fref.p, n, stream));
@@ -749,8 +739,7 @@ struct lbm_server {
         r->status = st;
         r->t_done = now();
         r->step_done = stats.steps;
-        r->fields.clear();
-        r->fields.shrink_to_fit();
+        r->fields.reset();
         if (st == LBM_ERR_CANCELLED) stats.cancelled++;
         else if (st != LBM_OK) stats.failed++;
         else stats.completed++;
@@ -819,8 +808,7 @@ struct lbm_server {
             init_solve(r, k);
             // pageable sources are staged when the copy call returns
             std::lock_guard<std::mutex> g(mu);
-            r->fields.clear();
-            r->fields.shrink_to_fit();
+            r->fields.reset();
             r->ps.flags.clear();
             r->ps.flags.shrink_to_fit();
         }
