@@ -78,6 +78,12 @@ struct HostSample {
     double residual = 1, resNorm = 0, initRes[100] = {0};
 };
 
+// whether no sample has a viscosity law (KArgs::constant_mu)
+inline bool constant_mu(const std::vector<SampleParams> &sp)
+{
+    return std::all_of(sp.begin(), sp.end(), [](const SampleParams &p) { return p.visc == 0; });
+}
+
 // What a sample needs on the device apart from its place in a packing.
 struct PreparedSample {
     SampleParams p{};  // offsets, first_tile and ntile are set when packed

@@ -53,7 +53,7 @@ struct SampleParams {
     // holds f - f_ref, h - h_ref with f_ref, h_ref the equilibria at
     // (rho0, 0, 0, T0); rho0 = shref = 0 (full storage) on the FP64 path.
     double rho0, T0n, shref;  // T0n = T0 / Tc
-    double inv_mu, two_over_bR;
+    double inv_mu, inv_Tc, two_over_bR;
     int wide;  // FP32 WENO5 weights in the range-safe form (see weno_face)
     double eps1;  // FP64: WENO5's epsilon for values not scaled by |e|, 1e-6 / c^2
     // ghost columns of the stage buffers (0 or GHOST_X): x-periodic samples
@@ -196,6 +196,20 @@ __device__ __forceinline__ float2 kc<float2>(double v) { return make_float2((flo
 template <>
 __device__ __forceinline__ double2 kc<double2>(double v) { return make_double2(v, v); }
 
+// FP64 reciprocal of a normal number: PTX's approximate reciprocal
+// (about 23 bits) and one third-order Newton (Chebyshev) step, y (1 + e + e^2)
+// with e = 1 - d y, whose error e^3 is below the FP64 rounding (measured: the
+// correctly rounded value or, rarely, its neighbour),
+// in a third of the operations of a division and without its branch for
+// special operands (a division per face was a fifth of the FP64 sweeps).
+__device__ __forceinline__ double rcp64(double d)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = __fma_rn(-d, y, 1.0);
+    return __fma_rn(y, __fma_rn(e, e, e), y);
+}
+
 // ------------------------------------------------------------ equilibria
 // equilibrium2D (cpuLBM.cpp:785-844) with the polynomials of
 // inlineFunctions.cpp:10-61, evaluated per symmetry family.  Normalised
@@ -211,13 +225,13 @@ struct EqState {
 };
 
 template <class C>
-__device__ __forceinline__ EqState<C> eq_state(double rho, double ux, double uy, double T, const SampleParams &sp)
+__device__ __forceinline__ EqState<C> eq_state(double rho, double ux, double uy, double Tn, const SampleParams &sp)
 {
     EqState<C> e;
     e.rho = (C)rho;
     e.u = (C)(ux * sp.inv_sRTc);
     e.v = (C)(uy * sp.inv_sRTc);
-    e.T = (C)(T / sp.Tc);
+    e.T = (C)Tn;
     e.K = (C)sp.K;
     e.rRTc = (C)(rho * sp.RTc);
     return e;
@@ -585,7 +599,12 @@ template <class C>
 struct EqArgs<C, false> {
     EqState<C> q;
     __device__ __forceinline__ EqArgs(double rho, double ux, double uy, double T, const SampleParams &sp)
-        : q(eq_state<C>(rho, ux, uy, T, sp)) {}
+        : q(eq_state<C>(rho, ux, uy, xmul(T, sp.inv_Tc), sp)) {}
+    // Ends the sharing of subexpressions between the families before and
+    // after it: kept for four families they are more registers than the few
+    // products that form them again are worth (RK3 stage 3 spilled 850 bytes
+    // a thread, 240 so).
+    __device__ __forceinline__ void part() { asm volatile("" : "+d"(q.u), "+d"(q.v), "+d"(q.T), "+d"(q.K)); }
     __device__ __forceinline__ void fam(int f, C *fe, C *he) const
     {
         if (f == 0) eq_fam0(q, fe[0], he[0]);
@@ -599,6 +618,7 @@ struct EqArgs<C, true> {
     EqDev<C> q;
     __device__ __forceinline__ EqArgs(double rho, double ux, double uy, double T, const SampleParams &sp)
         : q(eq_dev<C>(rho, ux, uy, T, sp)) {}
+    __device__ __forceinline__ void part() {}
     __device__ __forceinline__ void fam(int f, C *fe, C *he) const
     {
         if (f == 0) eqd_fam0(q, fe[0], he[0]);
@@ -629,6 +649,9 @@ struct Macro {
     double rho, ux, uy, T, p, q;
 };
 
+// LAW false: the samples have constant viscosity (no pow, whose call the
+// registers live across it would have to be saved for)
+template <bool LAW = true>
 __device__ __forceinline__ Macro macro_from_sums(double r, double rux, double ruy, double sh, const SampleParams &sp)
 {
     // stored deviations: add the rest state's rho0 and sum of h (0 when the
@@ -645,7 +668,7 @@ __device__ __forceinline__ Macro macro_from_sums(double r, double rux, double ru
     const double usq = __fma_rn(m.uy, m.uy, __dmul_rn(m.ux, m.ux));
     m.T = __dmul_rn(__fma_rn(sh, ir, __dmul_rn(-0.5, usq)), sp.two_over_bR);
     m.p = __dmul_rn(__dmul_rn(r, sp.R), m.T);
-    if (sp.visc == 0) {
+    if (!LAW || sp.visc == 0) {
         m.q = m.p * sp.inv_mu;  // 1/tau_f = p/mu
     } else {
         double mu = sp.mu * pow(m.T / sp.visc_T, sp.visc_exp);
@@ -736,16 +759,16 @@ __device__ __forceinline__ float rcp_approx(float d)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return r;
 }
-// the quotients of both lanes: FP32 by two reciprocals; FP64 by one division
-// of the product of the denominators (a division costs as much as ten
-// products; the products of two denominators stay far inside the FP64 range)
+// the quotients of both lanes: FP32 by two reciprocals; FP64 by one
+// reciprocal, of the product of the denominators (which stays far inside the
+// FP64 range)
 __device__ __forceinline__ float2 face_div(float2 n, float2 d)
 {
     return __fmul2_rn(n, make_float2(rcp_approx(d.x), rcp_approx(d.y)));
 }
 __device__ __forceinline__ double2 face_div(double2 n, double2 d)
 {
-    const double r = __drcp_rn(xmul(d.x, d.y));
+    const double r = rcp64(xmul(d.x, d.y));
     return make_double2(xmul(xmul(n.x, d.y), r), xmul(xmul(n.y, d.x), r));
 }
 

@@ -243,6 +243,7 @@ void prepare_sample(const HostSample &h, int prec, PreparedSample &out)
     p.dt = h.dt;
     p.c = h.c;
     p.inv_mu = 1.0 / h.mu;
+    p.inv_Tc = 1.0 / h.Tc;
     p.two_over_bR = 2.0 / (h.b * h.R);
     p.visc = h.mu_model;
     p.visc_exp = h.mu_model == 1 ? 0.5 + h.upsilon : 1.5;
@@ -652,6 +653,7 @@ struct lbm_batch {
         a.tmaps = d_maps.p;
         a.fref = d_fref.p;
         a.want_residual = want_res;
+        a.constant_mu = constant_mu(sp);
         a.eq_tol = 1e-6;
         return a;
     }

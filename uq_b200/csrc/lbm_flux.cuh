@@ -470,11 +470,39 @@ __host__ __device__ constexpr bool flux_early(int mode)
     return sizeof(S) == 8 || mode == 3;
 }
 
+// FP64, ahead of the block's barrier: everything that needs no flux.  v is the
+// state, and becomes the new value but for its flux term (RK3 stage 3: what
+// stage 3 relaxes from); m: the state's moment sums.  Whether the
+// equilibrium's mass check fails.
+template <int MODE, bool LAW>
+__device__ __forceinline__ bool flux_free(double2 (&v)[NQ], MomentSums &ms, const SampleParams &sp, double eq_tol)
+{
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) ms.add(i, v[i].x, v[i].y);
+    const Macro m = ms.macro<LAW>(sp);
+    EqArgs<double, false> q(m.rho, m.ux, m.uy, m.T, sp);
+    const std::conditional_t<MODE == 1, Stage3Base, Update<double, MODE>> u(m, sp);
+    double sf = 0;
+#pragma unroll
+    for (int fam = 0; fam < 4; ++fam) {
+        double fe[4], he[4];
+        q.part();
+        q.fam(fam, fe, he);
+#pragma unroll
+        for (int k = 0; k < (fam ? 4 : 1); ++k) {
+            const int i = fam ? 4 * fam - 3 + k : 0;
+            sf += fe[k];
+            v[i] = u.base(i, v[i], make_double2(fe[k], he[k]));
+        }
+    }
+    return MODE >= 4 && fabs(sf - m.rho) > eq_tol;
+}
+
 // The per-node half of a stencil phase (MODE as k_flux): the node's
 // divergences from its parts, then the RK3 stage 3 or the update.  The
 // block's barrier between the sweeps and this lies inside, after the loads
 // that do not depend on the sweeps.
-template <class S, int MODE, bool SWEEP, class PART>
+template <class S, int MODE, bool SWEEP, bool LAW, class PART>
 __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, const SampleParams &sp, const PART &part,
                                            const S *save, double *red, int TX, int NT, int tid)
 {
@@ -491,6 +519,8 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
     V *__restrict__ st = pair_base(a.state, sp) + o;
     C kx, ky;  // dt/dx, dt/dy (FP64: times |e|)
     V fv[NQ];  // the state (after RK3 stage 3: the update's partial sum)
+    bool bad = false, bad_eq = false;
+    MomentSums m0;  // FP64: the state's moment sums
     auto load = [&]() {
         const double cs = F32 ? 1.0 : sp.c;
         kx = (C)__dmul_rn(a.tdx[sp.xoff + x], cs);
@@ -501,7 +531,10 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
         }
     };
     if (EARLY) {
-        if (active) load();
+        if (active) {
+            load();
+            if constexpr (!F32 && MODE != 2) bad_eq = flux_free<MODE, LAW>(fv, m0, sp, a.eq_tol);
+        }
         __syncthreads();
     }
     pdl_trigger();
@@ -554,10 +587,43 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
             if (box_shape(i) == BOX_Y) return xmul(vy, part(i, 1));
             return xfma(vy, part(i, 1), xmul(vx, part(i, 0)));
         };
-        bool bad = false, bad_eq = false;
         MomentSums ms;           // of the new state, when the residual is wanted
         S fin_r = 0, fin_h = 0;  // NaN / Inf propagate through these sums as through FP64 ones
-        if constexpr (MODE == 1) {
+        if constexpr (MODE == 1 && !F32) {
+            // RK3 stage 3 and the part of the update that does not need the
+            // stage-3 fluxes, from the moments of f - div F(f2)
+            V *__restrict__ b3 = pair_base(a.buf3, sp) + o;
+#pragma unroll
+            for (int i = 1; i < NQ; ++i) {
+                const V D = div(i);
+                m0.sub(i, D.x, D.y);
+            }
+            const Macro m3 = m0.template macro<LAW>(sp);
+            EqArgs<C, DEV> q3(m3.rho, m3.ux, m3.uy, m3.T, sp);
+            const Stage3Rest s(m3, sp);
+            double sf3 = 0;
+#pragma unroll
+            for (int fam = 0; fam < 4; ++fam) {
+                C ef[4], eh[4];
+                asm volatile("" ::: "memory");  // (and the flux differences are read again)
+                q3.part();
+                q3.fam(fam, ef, eh);
+#pragma unroll
+                for (int k = 0; k < (fam ? 4 : 1); ++k) {
+                    const int i = fam ? 4 * fam - 3 + k : 0;
+                    sf3 += ef[k];
+                    V n3, acc;
+                    s.update(i, fv[i], div(i), make_pair2(ef[k], eh[k]), n3, acc);
+                    b3[i * PL] = n3;
+                    st[i * PL] = acc;
+                }
+            }
+            if (const int gd = ghost_offset(sp, x)) {
+#pragma unroll 1
+                for (int i = 0; i < NQ; ++i) b3[i * PL + gd] = b3[i * PL];
+            }
+            bad_eq = fabs(sf3 - m3.rho) > a.eq_tol;
+        } else if constexpr (MODE == 1) {
             // RK3 stage 3 (cpuLBM.cpp:1928-1993) and the part of the update
             // (cpuLBM.cpp:1999-2042) that does not need the stage-3 fluxes
             const V *__restrict__ b2 = pair_base(a.buf2, sp) + o;
@@ -567,20 +633,19 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
             MomentSums s1, s3;
 #pragma unroll
             for (int i = 0; i < NQ; ++i) {
-                const V v = EARLY ? fv[i] : st[i * PL];
+                const V v = st[i * PL];
                 const double f = (double)v.x, h = (double)v.y;
                 s1.add(i, f, h);
                 const V D = div(i);
                 s3.add(i, i ? __dsub_rn(f, (double)D.x) : f, i ? __dsub_rn(h, (double)D.y) : h);
             }
-            const Macro m1 = s1.macro(sp), m3 = s3.macro(sp);
+            const Macro m1 = s1.template macro<LAW>(sp), m3 = s3.template macro<LAW>(sp);
             const EqArgs<C, DEV> q1(m1.rho, m1.ux, m1.uy, m1.T, sp);
             const EqArgs<C, DEV> q3(m3.rho, m3.ux, m3.uy, m3.T, sp);
-            const Stage3<C> s(m1, m3, sp);
+            const Stage3 s(m1, m3, sp);
             double sf3 = 0;
             // family by family; the state is loaded a second time rather than
-            // kept (13 pairs of registers, which FP64 spilled and FP32 needs
-            // for the loads ahead)
+            // kept (13 pairs of registers, better used for the loads ahead)
             V gv[4], g2[4];
             auto fetch = [&](const int fam) {
                 const int i0 = fam == 0 ? 0 : 4 * fam - 3, n = fam == 0 ? 1 : 4;
@@ -588,7 +653,7 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
                 for (int k = 0; k < 4; ++k)
                     if (k < n) {
                         gv[k] = load_again(st + (i0 + k) * PL);
-                        if (F32) g2[k] = b2[(i0 + k) * PL];
+                        g2[k] = b2[(i0 + k) * PL];
                     }
             };
             auto family = [&](const int fam) {
@@ -602,7 +667,7 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
                     for (int k = 0; k < 4; ++k)
                         if (k < n) {
                             hv[k] = gv[k];
-                            d2[k] = s.dist(i0 + k, make_pair2(ef[k], eh[k]), hv[k], F32 ? g2[k] : kc<V>(0.0));
+                            d2[k] = xsub(make_pair2(ef[k], eh[k]), g2[k]);
                         }
                 }
                 C ef[4], eh[4];
@@ -628,19 +693,21 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
                 for (int i = 0; i < NQ; ++i) b3[i * PL + gd] = b3[i * PL];
             }
             bad_eq = fabs(sf3 - (m3.rho - sp.rho0)) > a.eq_tol * (sizeof(C) == 8 ? 1.0 : fmax(1.0, fabs(m3.rho)));
-        } else if constexpr (MODE == 2) {
-            // final RK3 combination (cpuLBM.cpp:1999-2042): f = acc - D3/2
+        } else if constexpr (MODE == 2 || !F32) {
+            // final RK3 combination (cpuLBM.cpp:1999-2042): f = acc - D3/2;
+            // the other updates' flux term
 #pragma unroll
             for (int i = 0; i < NQ; ++i) {
-                const V n = i ? xfma(kc<V>(-0.5), div(i), fv[i]) : fv[i];
-                if (i) st[i * PL] = n;
+                V n = fv[i];
+                if (i) n = MODE == 2 ? xfma(kc<V>(-0.5), div(i), n) : xsub(n, div(i));
+                if (i || MODE != 2) st[i * PL] = n;
                 fin_r += n.x;
                 fin_h += n.y;
                 if (a.want_residual) ms.add(i, (double)n.x, (double)n.y);
             }
         } else {
             // RK1 update (cpuLBM.cpp:1674-1710), EULER (:2130-2168), EULER_EQ (:2220-2258)
-            const Macro m = node_macro_rd([&](int i) { return fv[i]; }, sp);
+            const Macro m = node_macro_rd<LAW>([&](int i) { return fv[i]; }, sp);
             const EqArgs<C, DEV> q(m.rho, m.ux, m.uy, m.T, sp);
             const Update<C, MODE> u(m, sp);
             double sf = 0;
@@ -669,7 +736,7 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
             if (a.want_residual) {
                 // macroPropShort of the new state: the residual's T, and the
                 // finiteness / positive-density check
-                const Macro mn = ms.macro(sp);
+                const Macro mn = ms.template macro<false>(sp);  // (no relaxation time)
                 bad = !(mn.rho > 0.0) || !isfinite(mn.rho) || !isfinite(mn.T) || !isfinite(mn.ux) || !isfinite(mn.uy);
                 const double d = mn.T - a.told[sp.node_off + o];
                 res_part = d * d;
@@ -706,7 +773,7 @@ struct FluxBlocks {
 // block given the other kind returns at once).
 // TC: the default tile shape, compiled in; other shapes are read from the
 // arguments and give every node the same bits.
-template <class S, int MODE, int PATH, bool TC>
+template <class S, int MODE, int PATH, bool TC, bool LAW>
 __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP && TC>::value) k_flux(KArgs<S> a)
 {
     using V = Pair<S>;
@@ -816,7 +883,7 @@ __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP &&
                 }
         }
     }
-    node_phase<S, MODE, SWEEP>(a, s_tile, sp, part, save, red, TX, NT, tid);
+    node_phase<S, MODE, SWEEP, LAW>(a, s_tile, sp, part, save, red, TX, NT, tid);
 }
 
 // ----------------------------------------------------------------- launchers
@@ -844,9 +911,10 @@ cudaError_t launch_flux(int mode, const KArgs<S> &a, int ntiles, int path, cudaS
     cudaError_t e = cudaSuccess;
     with_mode(mode, [&](auto m) {
         constexpr int M = decltype(m)::value;
-        e = launch_step_kernel(!sweep ? k_flux<S, M, FLUX_GENERAL, false>
-                               : def  ? k_flux<S, M, FLUX_SWEEP, true>
-                                      : k_flux<S, M, FLUX_SWEEP, false>,
+        e = launch_step_kernel(!sweep ? k_flux<S, M, FLUX_GENERAL, false, true>
+                               : def  ? (k.constant_mu ? k_flux<S, M, FLUX_SWEEP, true, sizeof(S) == 4>
+                                                       : k_flux<S, M, FLUX_SWEEP, true, true>)
+                                      : k_flux<S, M, FLUX_SWEEP, false, true>,
                                ntiles, NT, sm, st, !k.phased, k);
     });
     return e;
@@ -863,9 +931,10 @@ cudaError_t prepare_flux()
     for (int mode = 1; mode <= 5; ++mode)
         with_mode(mode, [&](auto m) {
             constexpr int M = decltype(m)::value;
-            allow(k_flux<S, M, FLUX_GENERAL, false>);
-            allow(k_flux<S, M, FLUX_SWEEP, false>);
-            allow(k_flux<S, M, FLUX_SWEEP, true>);
+            allow(k_flux<S, M, FLUX_GENERAL, false, true>);
+            allow(k_flux<S, M, FLUX_SWEEP, false, true>);
+            allow(k_flux<S, M, FLUX_SWEEP, true, true>);
+            allow(k_flux<S, M, FLUX_SWEEP, true, sizeof(S) == 4>);
         });
     return e;
 }

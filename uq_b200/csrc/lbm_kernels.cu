@@ -32,7 +32,7 @@ template <class S>
 __device__ __noinline__ bool init_node(double rho, double ux, double uy, double T, const SampleParams &sp,
                                        const double *fr, S *state, S *buf2, S *buf3, long long o, bool fixed)
 {
-    EqState<double> q = eq_state<double>(rho, ux, uy, T, sp);
+    EqState<double> q = eq_state<double>(rho, ux, uy, T / sp.Tc, sp);
     double f[NQ], h[NQ];
     eq_all(q, f, h);
     double sf = 0;
@@ -59,7 +59,7 @@ template <class S>
 struct Stage0Blocks {
     static constexpr int value = sizeof(S) == 4 ? 3 : 2;
 };
-template <class S, int RK>
+template <class S, int RK, bool LAW>
 __global__ void __launch_bounds__(256, Stage0Blocks<S>::value) k_stage0(KArgs<S> a)
 {
     using C = S;
@@ -85,19 +85,20 @@ __global__ void __launch_bounds__(256, Stage0Blocks<S>::value) k_stage0(KArgs<S>
             b2[i * PL] = v[i];
             if (gd) b2[i * PL + gd] = v[i];
         }
-        if (a.want_residual) a.told[node] = node_macro_rd([&](int i) { return v[i]; }, sp).T;
+        if (a.want_residual) a.told[node] = node_macro_rd<false>([&](int i) { return v[i]; }, sp).T;
         return;
     }
-    const Macro m = node_macro_rd([&](int i) { return v[i]; }, sp);
+    const Macro m = node_macro_rd<LAW>([&](int i) { return v[i]; }, sp);
     pdl_trigger();
     if (a.want_residual) a.told[node] = m.T;
     constexpr bool DEV = sizeof(S) == 4;
-    const EqArgs<C, DEV> q(m.rho, m.ux, m.uy, m.T, sp);
+    EqArgs<C, DEV> q(m.rho, m.ux, m.uy, m.T, sp);
     const PointStage<C, RK == 1 ? 1 : 0> p(m, sp);
     double sf = 0;
 #pragma unroll
     for (int fam = 0; fam < 4; ++fam) {
         C fe[4], he[4];
+        q.part();
         q.fam(fam, fe, he);
         const int i0 = fam == 0 ? 0 : 4 * fam - 3, n = fam == 0 ? 1 : 4;
 #pragma unroll
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(256, Stage0Blocks<S>::value) k_stage0(KArgs<S>
             if (k >= n) break;
             const int i = i0 + k;
             sf += (double)fe[k];
-                        const V nv = p.value(i, v[i], make_pair2(fe[k], he[k]));
+            const V nv = p.value(i, v[i], make_pair2(fe[k], he[k]));
             b2[i * PL] = nv;
             if (gd) b2[i * PL + gd] = nv;
         }
@@ -362,7 +363,10 @@ cudaError_t launch_phase(const KArgs<S> &a, int phase, int rk, const Tile *tiles
     const int NT = a.tx * a.ty;
     if (phase == 0) {
         if (!ntiles) return cudaSuccess;
-        return launch_step_kernel(rk == 1 ? k_stage0<S, 1> : rk == 0 ? k_stage0<S, 0> : k_stage0<S, 2>, ntiles, NT, 0, st,
+        return launch_step_kernel(rk >= 2         ? k_stage0<S, 2, false>
+                                  : k.constant_mu ? (rk ? k_stage0<S, 1, sizeof(S) == 4> : k_stage0<S, 0, sizeof(S) == 4>)
+                                                  : (rk ? k_stage0<S, 1, true> : k_stage0<S, 0, true>),
+                                  ntiles, NT, 0, st,
                                   !k.phased, k);
     } else if (phase == 1 || phase == 2) {
         if (!ntiles) return cudaSuccess;

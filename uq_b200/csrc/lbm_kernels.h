@@ -53,6 +53,7 @@ struct KArgs {
     // the ghost columns to k_fill_ghosts, and straight walls take their
     // factors from k_wall
     int phased;
+    int constant_mu;  // no sample has a viscosity law
     double eq_tol;
 #ifdef __CUDACC__
     // alpha is stored in the compute type of the kernel instantiation

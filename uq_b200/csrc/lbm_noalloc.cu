@@ -230,6 +230,7 @@ static lbm_status step_noalloc(const lbm_config *cfg, int Nx, int Ny, const int 
     sp.dt = sc.dt;
     sp.c = sc.c;
     sp.inv_mu = 1.0 / sc.mu;
+    sp.inv_Tc = 1.0 / sc.Tc;
     sp.eps1 = std::min(std::max(1e-6 / (sc.c * sc.c), 1e-35), 1e35);
     sp.two_over_bR = 2.0 / (sc.b * sc.R);
     sp.visc = sc.mu_model;
@@ -287,6 +288,7 @@ static lbm_status step_noalloc(const lbm_config *cfg, int Nx, int Ny, const int 
     a.tmaps = reinterpret_cast<const CUtensorMap *>(base + NA_OFF_MAPS);
     a.fref = reinterpret_cast<const double *>(base + NA_OFF_FREF);
     a.want_residual = 0;
+    a.constant_mu = sc.mu_model == 0;
     a.eq_tol = 1e-6;
     TileRun sweep, general;
     split_runs(a.tiles, sp.ntile, ns, sweep, general);

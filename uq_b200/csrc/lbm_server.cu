@@ -156,6 +156,7 @@ struct lbm_server {
     std::vector<double> v_tdx, v_tdy, v_dx, v_dy, v_fref;
     std::vector<CUtensorMap> maps;
     DevBuf<SampleParams> d_sp;
+    bool const_mu = true;  // of the packed solves
     DevBuf<Tile> d_tiles_rk3, d_tiles_by_rk[4], d_flux_by_rk[4];
     DevBuf<WallNode> d_walls_all, d_walls_rk3;
     DevBuf<double> d_tdx, d_tdy, d_dx, d_dy, d_fref;
@@ -401,6 +402,7 @@ struct lbm_server {
         }
         tiles_rk3.insert(tiles_rk3.end(), gen_rk3.begin(), gen_rk3.end());
         d_sp.upload_keep(sp, stream);
+        const_mu = constant_mu(sp);
         for (int m = 0; m < 4; ++m) {
             d_tiles_by_rk[m].upload_keep(tiles_by_rk[m], stream);
             d_flux_by_rk[m].upload_keep(flux_by_rk[m], stream);
@@ -479,6 +481,7 @@ struct lbm_server {
         a.tmaps = d_maps.p;
         a.fref = d_fref.p;
         a.want_residual = 0;
+        a.constant_mu = const_mu;
         a.eq_tol = 1e-6;
         return a;
     }
