@@ -55,7 +55,7 @@ struct FluxSmem {
     int slots;       // boxes resident at a time
     int slot_pairs;  // pairs per slot (not the default tile)
     int part_off;    // the parts (default tile: the diagonals' x parts), in pairs
-    int wall_off;    // saved wall faces, in pairs
+    int wall_off;    // saved wall faces (general tiles: faces into the tile), in pairs
     int bar_off;     // mbarriers, in pairs
     size_t bytes;    // with 128 bytes of base-alignment slack
 };
@@ -92,7 +92,8 @@ __host__ __device__ constexpr FluxSmem flux_smem(int tx, int ty, bool def, bool 
         off += 16 * part_pairs(tx, ty);
     }
     L.wall_off = off;
-    if (sweep) off += (4 * tx + 15) / 16 * 16;  // [2 walls][4][tx] values of S
+    // [2 walls][4][tx] values of S; general tiles: the faces into the tile
+    off += sweep ? (4 * tx + 15) / 16 * 16 : 8 * (tx + ty);
     L.bar_off = off;
     L.bytes = (size_t)off * pb + 12 * sizeof(uint64_t) + 128;
     return L;
@@ -418,6 +419,66 @@ __device__ __noinline__ Pair<S> node_face(const SampleParams &sp, const StageVie
     if ((fl & NF_TYPE) == 2)
         return wall_flux<S>(alpha[o], ldv(v, i, x, y), fref, i, face_arg<S>(sp, axis == 0 ? c_EX[i] : c_EY[i]));
     return flux_axis<S, S>(sp, v, x, y, i, axis, fl);
+}
+
+// the a-th direction (0..7) that moves along an axis
+__host__ __device__ constexpr int moving(int a, int axis) { return a < 2 ? 1 + 2 * a + axis : a < 6 ? a + 3 : 2 * a - 3 + axis; }
+
+// General tiles: every face once.  Each thread answers the faces of its own
+// node; those that enter the tile from outside (the upstream node wrapped,
+// clamped or, at a mirror edge, of the reflected direction) are shared out
+// over the block's threads.  The faces' arithmetic bounds these tiles, not
+// memory: a 1024^2 step with 64 obstacles took 0.770 ms (FP64 1.051) with two
+// faces per node, axis and direction, 0.621 (0.860) with one.
+template <class S>
+__device__ __forceinline__ void face_parts(const Tile &t, const SampleParams &sp, const StageView<S> &v, const S *alpha,
+                                           const double *fref, Pair<S> *parts, Pair<S> *edges, int TX, int TY, int tid,
+                                           int NT)
+{
+    using V = Pair<S>;
+    const int PR = TX + 1, PP = part_pairs(TX, TY), tx = tid % TX, ty = tid / TX, pn = ty * PR + tx;
+    const int x = t.x0 + tx, y = t.y0 + ty, xe = min(t.x0 + TX, sp.nx), ye = min(t.y0 + TY, sp.ny);
+    const bool in = x < xe && y < ye;
+    if (in) {
+#pragma unroll 1
+        for (int k = 0; k < 16; ++k) {
+            const int axis = k >> 3, i = moving(k & 7, axis);
+            parts[part_index(i, axis) * PP + pn] = node_face<S>(sp, v, alpha, fref, i, axis, x, y);
+        }
+    }
+#pragma unroll 1
+    for (int k = tid; k < 8 * (TX + TY); k += NT) {
+        const int axis = k >= 8 * TY, r = axis ? k - 8 * TY : k, n = axis ? TX : TY;
+        const int i = moving(r / n, axis), e = axis ? c_EY[i] : c_EX[i], j = r % n;
+        // the tile's first node downstream of the face
+        const int fx = axis ? t.x0 + j : e > 0 ? t.x0 : xe - 1, fy = axis ? (e > 0 ? t.y0 : ye - 1) : t.y0 + j;
+        if (fx >= xe || fy >= ye || (v.nf[fy * v.pitch + fx] & NF_TYPE) != 0) continue;
+        int m;
+        const int u = bc_index(sp, axis ? fy : fx, e > 0 ? -1 : 1, axis, m);
+        const int iu = m ? (axis ? c_MIR_NS[i] : c_MIR_EW[i]) : i;
+        edges[k] = node_face<S>(sp, v, alpha, fref, iu, axis, axis ? fx : u, axis ? u : fy);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int axis = 0; axis < 2; ++axis) {
+        V d[8];
+        if (in) {
+#pragma unroll
+            for (int a = 0; a < 8; ++a) {
+                const int i = moving(a, axis), up = (axis ? lat_ey(i) : lat_ex(i)) > 0 ? -1 : 1;
+                const int first = axis ? (up < 0 ? t.y0 : ye - 1) : up < 0 ? t.x0 : xe - 1;
+                const V *p = parts + part_index(i, axis) * PP + pn;
+                const V *q = (axis ? y : x) != first ? p + up * (axis ? PR : 1)
+                                                     : edges + (axis ? 8 * TY + a * TX + tx : a * TY + ty);
+                d[a] = xsub(*p, *q);
+            }
+        }
+        __syncthreads();
+        if (in) {
+#pragma unroll
+            for (int a = 0; a < 8; ++a) parts[part_index(moving(a, axis), axis) * PP + pn] = d[a];
+        }
+    }
 }
 
 // the whole block of a default tile: each warp its directions
@@ -861,27 +922,9 @@ __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP &&
     const int tx = tid % TX, ty = tid / TX;
     const NodeParts<S, TC && SWEEP> part{TC && SWEEP ? sm : sm + L.part_off, ty * PR + tx, PP};
     if constexpr (!SWEEP) {
-        const int x = t.x0 + tx, y = t.y0 + ty;
-        if (x < sp.nx && y < sp.ny && (a.nflags[sp.node_off + y * sp.pitch + x] & NF_TYPE) == 0) {
-            const StageView<S> v{stage + sp.state_off, a.nflags + sp.node_off, (int)sp.plane, sp.pitch};
-            const S *alpha = a.template alpha_as<S>() + sp.node_off;
-            const double *fr = a.fref + NPL * t.sample;
-#pragma unroll 1
-            for (int i = 1; i < NQ; ++i)
-#pragma unroll 1
-                for (int axis = 0; axis < 2; ++axis) {
-                    const int e = isgn(axis == 0 ? c_EX[i] : c_EY[i]);
-                    if (e == 0) continue;
-                    // upstream face: index(x, -e), reflected at a mirror edge
-                    int m;
-                    const int u = bc_index(sp, axis == 0 ? x : y, -e, axis, m);
-                    const int iu = m ? (axis == 0 ? c_MIR_EW[i] : c_MIR_NS[i]) : i;
-                    const V out = node_face<S>(sp, v, alpha, fr, i, axis, x, y);
-                    const V in = axis == 0 ? node_face<S>(sp, v, alpha, fr, iu, 0, u, y)
-                                           : node_face<S>(sp, v, alpha, fr, iu, 1, x, u);
-                    part(i, axis) = xsub(out, in);
-                }
-        }
+        const StageView<S> v{stage + sp.state_off, a.nflags + sp.node_off, (int)sp.plane, sp.pitch};
+        face_parts<S>(t, sp, v, a.template alpha_as<S>() + sp.node_off, a.fref + NPL * t.sample, sm + L.part_off,
+                      sm + L.wall_off, TX, TY, tid, NT);
     }
     node_phase<S, MODE, SWEEP, LAW>(a, s_tile, sp, part, save, red, TX, NT, tid);
 }
