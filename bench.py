@@ -751,7 +751,7 @@ def run_ours(args, rank, world, local_rank):
                          "wall)" % (cores, "/".join(str(REF_SIDE_STEPS[x]) for x in sorted(REF_SIDE_STEPS)), wall),
                **detail}
 
-    launches = b.graph_launches(False) * args.steps
+    launches = b.step_launches(args.steps)
     b.close()
     if rank == 0 and world == 1 and args.serving_seconds > 0 and not args.no_probes:
         try:

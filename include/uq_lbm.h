@@ -247,8 +247,9 @@ LBM_API lbm_status lbm_batch_autotune(lbm_batch *b, const int *candidates, int n
 /* Kernel launches of one step taken phase by phase, every part apart: what
  * lbm_batch_profile times and a batch without use_graph runs ... */
 LBM_API int lbm_batch_launches_per_step(lbm_batch *b, int want_residual);
-/* ... and of one step replayed from a graph, which merges the parts. */
-LBM_API int lbm_batch_graph_launches(lbm_batch *b, int want_residual);
+/* Kernel launches of lbm_batch_step(b, n, want_residual): with use_graph the
+ * parts are merged, and steps in a row share launches. */
+LBM_API long long lbm_batch_step_launches(lbm_batch *b, int n, int want_residual);
 /* Lattice updates (nodes) one step of the whole batch performs. */
 LBM_API long long lbm_batch_nodes(lbm_batch *b);
 LBM_API void *lbm_batch_stream(lbm_batch *b);

@@ -167,30 +167,35 @@ void stencil_runs(const KArgs<S> &a, int phase, int m, const TileRun &s, const T
     if (g.n) CU((launch_phase<S, C>(a, phase, m, g.p, g.n, nullptr, 0, st, FLUX_GENERAL)));
 }
 
-// One step: pointwise stages, first stencil phase, and for RK3 the final
+// n steps: pointwise stages, first stencil phase, and for RK3 the final
 // stencil phase; wall factors before a stencil phase with general tiles that
-// read some.
+// read some.  Where steps are joined, RK3's final phase forms the next step's
+// pointwise stages, so that only the first step launches them.
 template <class S, class C>
-void enqueue_step(const KArgs<S> &a, const StepLists &l, cudaStream_t st)
+void enqueue_steps(KArgs<S> a, const StepLists &l, int n, cudaStream_t st)
 {
-    for (int m = 0; m < 4; ++m)
-        if (l.pointwise[m].n) CU((launch_phase<S, C>(a, 0, m, l.pointwise[m].p, l.pointwise[m].n, nullptr, 0, st)));
-    CU((launch_phase<S, C>(a, 3, 0, nullptr, 0, l.walls_all, l.n_walls_all, st)));
-    for (int m = 0; m < 4; ++m) stencil_runs<S, C>(a, 1, m, l.sweep[m], l.general[m], st);
-    if (l.rk3_sweep.n || l.rk3_general.n) {
+    const bool join = joins<S>(a.tx, a.ty);
+    const bool rk3 = l.rk3_sweep.n || l.rk3_general.n;
+    for (int k = 0; k < n; ++k) {
+        for (int m = 0; m < 4; ++m)
+            if (l.pointwise[m].n && !(join && m == 1 && k)) CU((launch_phase<S, C>(a, 0, m, l.pointwise[m].p, l.pointwise[m].n, nullptr, 0, st)));
+        CU((launch_phase<S, C>(a, 3, 0, nullptr, 0, l.walls_all, l.n_walls_all, st)));
+        for (int m = 0; m < 4; ++m) stencil_runs<S, C>(a, 1, m, l.sweep[m], l.general[m], st);
+        if (!rk3) continue;
         CU((launch_phase<S, C>(a, 4, 1, nullptr, 0, l.walls_rk3, l.n_walls_rk3, st)));
+        a.next = join && k + 1 < n;
         stencil_runs<S, C>(a, 2, 1, l.rk3_sweep, l.rk3_general, st);
     }
 }
 
-// kernels that enqueue_step launches
-inline int step_launches(const StepLists &l)
+// kernels that enqueue_steps launches
+inline int steps_launches(const StepLists &l, int n, bool join)
 {
-    int n = l.n_walls_all ? 1 : 0;
-    for (int m = 0; m < 4; ++m) n += (l.pointwise[m].n ? 1 : 0) + (l.sweep[m].n ? 1 : 0) + (l.general[m].n ? 1 : 0);
+    int per = l.n_walls_all ? 1 : 0;
+    for (int m = 0; m < 4; ++m) per += (l.pointwise[m].n ? 1 : 0) + (l.sweep[m].n ? 1 : 0) + (l.general[m].n ? 1 : 0);
     if (l.rk3_sweep.n || l.rk3_general.n)
-        n += (l.n_walls_rk3 ? 1 : 0) + (l.rk3_sweep.n ? 1 : 0) + (l.rk3_general.n ? 1 : 0);
-    return n;
+        per += (l.n_walls_rk3 ? 1 : 0) + (l.rk3_sweep.n ? 1 : 0) + (l.rk3_general.n ? 1 : 0);
+    return n * per - (join && n > 0 && l.pointwise[1].n ? n - 1 : 0);
 }
 
 // The same step phase by phase, every part in launches of its own (the ghost

@@ -786,17 +786,26 @@ struct lbm_batch {
     // 7 events around the phases: [0] start, then after pointwise, walls 2,
     // phase 1, walls 3, phase 2, residual.
     template <class S, class C>
-    void enqueue_step_t(int want_res, bool phased, cudaEvent_t *ev = nullptr)
+    void enqueue_step_t(int want_res, bool phased, int n, cudaEvent_t *ev = nullptr)
     {
         if (phased) enqueue_step_phased<S, C>(args<S>(want_res), lists(), stream, ev);
-        else uqlbm::enqueue_step<S, C>(args<S>(want_res), lists(), stream);
+        else enqueue_steps<S, C>(args<S>(want_res), lists(), n, stream);
         if (want_res)
             CU(launch_residual(d_sp.p, (int)hs.size(), partial.p, d_tile_first.p, d_tile_count.p, residual.p, stream));
         if (ev) CU(cudaEventRecord(ev[6], stream));
     }
 
     int launches_per_step(int want_res) const { return phased_launches(lists()) + (want_res ? 1 : 0); }
-    int graph_launches(int want_res) const { return step_launches(lists()) + (want_res ? 1 : 0); }
+    // kernels of launch_steps(n, want_res)
+    long long step_launches(int n, int want_res) const
+    {
+        if (!use_graph) return (long long)n * launches_per_step(want_res);
+        const StepLists l = lists();
+        const bool join = prec == LBM_PREC_F32 && joins<float>(tx, ty);
+        const int runs = want_res ? 0 : n / kGraphSteps;
+        return (long long)runs * steps_launches(l, kGraphSteps, join)
+             + (long long)(n - runs * kGraphSteps) * (steps_launches(l, 1, join) + (want_res ? 1 : 0));
+    }
 
     void profile(int n, double *ms, int nph)
     {
@@ -804,8 +813,8 @@ struct lbm_batch {
         for (auto &e : ev) CU(cudaEventCreate(&e));
         std::vector<double> acc(6, 0.0);
         for (int k = 0; k < n; ++k) {
-            if (prec == LBM_PREC_F64) enqueue_step_t<double, double>(1, true, ev);
-            else enqueue_step_t<float, float>(1, true, ev);
+            if (prec == LBM_PREC_F64) enqueue_step_t<double, double>(1, true, 1, ev);
+            else enqueue_step_t<float, float>(1, true, 1, ev);
             CU(cudaEventSynchronize(ev[6]));
             for (int p = 0; p < 6; ++p) {
                 float t = 0;
@@ -893,10 +902,11 @@ struct lbm_batch {
         CU(cudaStreamSynchronize(stream));
     }
 
-    void enqueue_step(int want_res)
+    // (n > 1: from a graph, without the residual)
+    void enqueue_step(int want_res, int n = 1)
     {
-        if (prec == LBM_PREC_F64) enqueue_step_t<double, double>(want_res, !use_graph);
-        else enqueue_step_t<float, float>(want_res, !use_graph);
+        if (prec == LBM_PREC_F64) enqueue_step_t<double, double>(want_res, !use_graph, n);
+        else enqueue_step_t<float, float>(want_res, !use_graph, n);
     }
 
     void launch_steps(int n, int want_res)
@@ -916,7 +926,7 @@ struct lbm_batch {
         cudaGraph_t gr;
         CU(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         try {
-            for (int k = 0; k < (g == 2 ? kGraphSteps : 1); ++k) enqueue_step(g == 1);
+            enqueue_step(g == 1, g == 2 ? kGraphSteps : 1);
         } catch (...) {
             cudaStreamEndCapture(stream, &gr);
             throw;
@@ -1380,7 +1390,10 @@ lbm_status lbm_batch_autotune(lbm_batch *b, const int *candidates, int n_candida
 
 int lbm_batch_launches_per_step(lbm_batch *b, int want_residual) { return b ? b->launches_per_step(want_residual) : 0; }
 
-int lbm_batch_graph_launches(lbm_batch *b, int want_residual) { return b ? b->graph_launches(want_residual) : 0; }
+long long lbm_batch_step_launches(lbm_batch *b, int n, int want_residual)
+{
+    return b && n > 0 ? b->step_launches(n, want_residual) : 0;
+}
 
 lbm_status lbm_batch_set_dist(lbm_batch *b, int sample, const double *f, const double *hh)
 {

@@ -563,7 +563,7 @@ __device__ __forceinline__ bool flux_free(double2 (&v)[NQ], MomentSums &ms, cons
 // divergences from its parts, then the RK3 stage 3 or the update.  The
 // block's barrier between the sweeps and this lies inside, after the loads
 // that do not depend on the sweeps.
-template <class S, int MODE, bool SWEEP, bool LAW, class PART>
+template <class S, int MODE, bool SWEEP, bool LAW, bool NEXT, class PART>
 __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, const SampleParams &sp, const PART &part,
                                            const S *save, double *red, int TX, int NT, int tid)
 {
@@ -762,9 +762,10 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
                 V n = fv[i];
                 if (i) n = MODE == 2 ? xfma(kc<V>(-0.5), div(i), n) : xsub(n, div(i));
                 if (i || MODE != 2) st[i * PL] = n;
+                if (NEXT) fv[i] = n;
                 fin_r += n.x;
                 fin_h += n.y;
-                if (a.want_residual) ms.add(i, (double)n.x, (double)n.y);
+                if (NEXT || a.want_residual) ms.add(i, (double)n.x, (double)n.y);
             }
         } else {
             // RK1 update (cpuLBM.cpp:1674-1710), EULER (:2130-2168), EULER_EQ (:2220-2258)
@@ -793,8 +794,18 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
             if (MODE >= 4)
                 bad_eq = fabs(sf - (m.rho - sp.rho0)) > a.eq_tol * (sizeof(C) == 8 ? 1.0 : fmax(1.0, fabs(m.rho)));
         }
+        if constexpr (NEXT) {
+            // the next step's stages 1 and 2, into the buffer that this
+            // phase does not read
+            V *__restrict__ b2 = pair_base(a.buf2, sp) + o;
+            bad_eq = first_stage<S, 1>(fv, ms.template macro<LAW>(sp), sp, a.eq_tol, [&](int i, V nv) { b2[i * PL] = nv; });
+            if (const int gd = ghost_offset(sp, x)) {
+#pragma unroll 1
+                for (int i = 0; i < NQ; ++i) b2[i * PL + gd] = b2[i * PL];
+            }
+        }
         if (MODE != 1) {
-            if (a.want_residual) {
+            if (!NEXT && a.want_residual) {
                 // macroPropShort of the new state: the residual's T, and the
                 // finiteness / positive-density check
                 const Macro mn = ms.template macro<false>(sp);  // (no relaxation time)
@@ -809,7 +820,7 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
         if (bad_eq) atomicOr(&a.status[t.sample], STATUS_EQ);
         if (bad) atomicOr(&a.status[t.sample], STATUS_NONFINITE);
     }
-    if (a.want_residual && MODE != 1) {
+    if (!NEXT && a.want_residual && MODE != 1) {
         // per-tile partial sum, fixed order (deterministic)
         for (int off = 16; off > 0; off >>= 1) res_part += __shfl_down_sync(0xffffffffu, res_part, off);
         if ((tid & 31) == 0) red[tid >> 5] = res_part;
@@ -834,7 +845,7 @@ struct FluxBlocks {
 // block given the other kind returns at once).
 // TC: the default tile shape, compiled in; other shapes are read from the
 // arguments and give every node the same bits.
-template <class S, int MODE, int PATH, bool TC, bool LAW>
+template <class S, int MODE, int PATH, bool TC, bool LAW, bool NEXT>
 __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP && TC>::value) k_flux(KArgs<S> a)
 {
     using V = Pair<S>;
@@ -926,7 +937,7 @@ __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP &&
         face_parts<S>(t, sp, v, a.template alpha_as<S>() + sp.node_off, a.fref + NPL * t.sample, sm + L.part_off,
                       sm + L.wall_off, TX, TY, tid, NT);
     }
-    node_phase<S, MODE, SWEEP, LAW>(a, s_tile, sp, part, save, red, TX, NT, tid);
+    node_phase<S, MODE, SWEEP, LAW, NEXT>(a, s_tile, sp, part, save, red, TX, NT, tid);
 }
 
 // ----------------------------------------------------------------- launchers
@@ -943,23 +954,31 @@ void with_mode(int mode, F f)
     }
 }
 
+// calls f with every instance that launch_flux can take
+template <class S, class F>
+void with_kernel(int mode, bool sweep, bool def, bool constant_mu, bool next, F f)
+{
+    with_mode(mode, [&](auto m) {
+        constexpr int M = decltype(m)::value;
+        constexpr bool NX = M == 2 && joins<S>(TILE_CX, TILE_CY);
+        constexpr bool L0 = sizeof(S) == 4;
+        if (sweep && !def) f(k_flux<S, M, FLUX_SWEEP, false, true, false>);
+        else if (!sweep) f(next ? k_flux<S, M, FLUX_GENERAL, false, true, NX> : k_flux<S, M, FLUX_GENERAL, false, true, false>);
+        else if (next) f(constant_mu ? k_flux<S, M, FLUX_SWEEP, true, L0, NX> : k_flux<S, M, FLUX_SWEEP, true, true, NX>);
+        else f(constant_mu ? k_flux<S, M, FLUX_SWEEP, true, L0, false> : k_flux<S, M, FLUX_SWEEP, true, true, false>);
+    });
+}
+
 template <class S>
 cudaError_t launch_flux(int mode, const KArgs<S> &a, int ntiles, int path, cudaStream_t st)
 {
     KArgs<S> k = a;
     const bool def = k.tx == TILE_CX && k.ty == TILE_CY, sweep = path == FLUX_SWEEP;
     k.slots = def ? 12 : flux_slots<S>(k.tx, k.ty);
-    const int NT = k.tx * k.ty;
     const size_t sm = flux_smem_bytes_t<S>(k.tx, k.ty, sweep);
     cudaError_t e = cudaSuccess;
-    with_mode(mode, [&](auto m) {
-        constexpr int M = decltype(m)::value;
-        e = launch_step_kernel(!sweep ? k_flux<S, M, FLUX_GENERAL, false, true>
-                               : def  ? (k.constant_mu ? k_flux<S, M, FLUX_SWEEP, true, sizeof(S) == 4>
-                                                       : k_flux<S, M, FLUX_SWEEP, true, true>)
-                                      : k_flux<S, M, FLUX_SWEEP, false, true>,
-                               ntiles, NT, sm, st, !k.phased, k);
-    });
+    with_kernel<S>(mode, sweep, def, k.constant_mu, k.next,
+                   [&](auto *kernel) { e = launch_step_kernel(kernel, ntiles, k.tx * k.ty, sm, st, !k.phased, k); });
     return e;
 }
 
@@ -968,17 +987,11 @@ cudaError_t prepare_flux()
 {
     const int maxsm = 224 * 1024;
     cudaError_t e = cudaSuccess;
-    auto allow = [&](auto *kernel) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm);
-    };
     for (int mode = 1; mode <= 5; ++mode)
-        with_mode(mode, [&](auto m) {
-            constexpr int M = decltype(m)::value;
-            allow(k_flux<S, M, FLUX_GENERAL, false, true>);
-            allow(k_flux<S, M, FLUX_SWEEP, false, true>);
-            allow(k_flux<S, M, FLUX_SWEEP, true, true>);
-            allow(k_flux<S, M, FLUX_SWEEP, true, sizeof(S) == 4>);
-        });
+        for (int k = 0; k < 16; ++k)
+            with_kernel<S>(mode, k & 1, k & 2, k & 4, k & 8, [&](auto *kernel) {
+                if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm);
+            });
     return e;
 }
 

@@ -91,29 +91,11 @@ __global__ void __launch_bounds__(256, Stage0Blocks<S>::value) k_stage0(KArgs<S>
     const Macro m = node_macro_rd<LAW>([&](int i) { return v[i]; }, sp);
     pdl_trigger();
     if (a.want_residual) a.told[node] = m.T;
-    constexpr bool DEV = sizeof(S) == 4;
-    EqArgs<C, DEV> q(m.rho, m.ux, m.uy, m.T, sp);
-    const PointStage<C, RK == 1 ? 1 : 0> p(m, sp);
-    double sf = 0;
-#pragma unroll
-    for (int fam = 0; fam < 4; ++fam) {
-        C fe[4], he[4];
-        q.part();
-        q.fam(fam, fe, he);
-        const int i0 = fam == 0 ? 0 : 4 * fam - 3, n = fam == 0 ? 1 : 4;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (k >= n) break;
-            const int i = i0 + k;
-            sf += (double)fe[k];
-            const V nv = p.value(i, v[i], make_pair2(fe[k], he[k]));
-            b2[i * PL] = nv;
-            if (gd) b2[i * PL + gd] = nv;
-        }
-    }
-    // sum_i f_eq = rho (the stored values: sum = rho - rho0)
-    if (fabs(sf - (m.rho - sp.rho0)) > a.eq_tol * (sizeof(C) == 8 ? 1.0 : fmax(1.0, fabs(m.rho))))
-        atomicOr(&a.status[t.sample], STATUS_EQ);
+    const bool bad = first_stage<S, RK == 1 ? 1 : 0>(v, m, sp, a.eq_tol, [&](int i, V nv) {
+        b2[i * PL] = nv;
+        if (gd) b2[i * PL + gd] = nv;
+    });
+    if (bad) atomicOr(&a.status[t.sample], STATUS_EQ);
 }
 
 // -------------------------------------------------------------------- W

@@ -25,6 +25,18 @@ constexpr int MAPS_PER_SAMPLE = 6;
 // of one direction along either axis are one warp's work (see lbm_flux.cuh).
 constexpr int TILE_CX = 32, TILE_CY = 8;
 
+// Whether RK3 steps in a row are joined (the final phase of one forms stages 1
+// and 2 of the next: the state is not read again, 104 of 936 bytes a node).
+// FP32 gains 3 % on large batches and nothing on the smallest.  FP64 would
+// gain 2 % and lose 6 % at 64 x 128, where the longer kernel is a longer
+// chain; RK1 has one stencil phase, which would have to fill a buffer that it
+// does not read, and loses 5 % to spills.
+template <class S>
+constexpr bool joins(int tx, int ty)
+{
+    return sizeof(S) == 4 && tx == TILE_CX && ty == TILE_CY;
+}
+
 struct WallNode {
     int sample, x, y, pad;
 };
@@ -53,6 +65,8 @@ struct KArgs {
     // the ghost columns to k_fill_ghosts, and straight walls take their
     // factors from k_wall
     int phased;
+    // RK3's final phase also forms the next step's stages 1 and 2
+    int next;
     int constant_mu;  // no sample has a viscosity law
     double eq_tol;
 #ifdef __CUDACC__

@@ -202,6 +202,32 @@ struct PointStage<double, RK> {
     }
 };
 
+// The pointwise stage that a step begins with, of a node with state v and
+// moments m: RK3's stages 1 and 2 (RK 1) or RK1's stage 1 (RK 0), each value
+// given to store(i, value).  Whether the equilibrium's mass check
+// (sum f_eq = rho, in the stored values rho - rho0) fails.
+template <class C, int RK, class STORE>
+__device__ __forceinline__ bool first_stage(const Pair<C> (&v)[NQ], const Macro &m, const SampleParams &sp, double eq_tol,
+                                            STORE store)
+{
+    EqArgs<C, sizeof(C) == 4> q(m.rho, m.ux, m.uy, m.T, sp);
+    const PointStage<C, RK> p(m, sp);
+    double sf = 0;
+#pragma unroll
+    for (int fam = 0; fam < 4; ++fam) {
+        C fe[4], he[4];
+        q.part();
+        q.fam(fam, fe, he);
+#pragma unroll
+        for (int k = 0; k < (fam ? 4 : 1); ++k) {
+            const int i = fam ? 4 * fam - 3 + k : 0;
+            sf += (double)fe[k];
+            store(i, p.value(i, v[i], make_pair2(fe[k], he[k])));
+        }
+    }
+    return fabs(sf - (m.rho - sp.rho0)) > eq_tol * (sizeof(C) == 8 ? 1.0 : fmax(1.0, fabs(m.rho)));
+}
+
 // RK3 stage 3 (cpuLBM.cpp:1928-1993) and the part of the update
 // (cpuLBM.cpp:1999-2042) that does not need the stage-3 fluxes, of direction
 // i: from the state v, the divergence D of stage 2's fluxes, and the

@@ -491,13 +491,11 @@ struct lbm_server {
     void enqueue_one_step()
     {
         if (prec == LBM_PREC_F64) {
-            enqueue_step<double, double>(args<double>(), lists, stream);
-            for (int j = 1; n_fast && j < fast_k; ++j)
-                enqueue_step<double, double>(args<double>(), fast_lists, stream);
+            enqueue_steps<double, double>(args<double>(), lists, 1, stream);
+            if (n_fast) enqueue_steps<double, double>(args<double>(), fast_lists, fast_k - 1, stream);
         } else {
-            enqueue_step<float, float>(args<float>(), lists, stream);
-            for (int j = 1; n_fast && j < fast_k; ++j)
-                enqueue_step<float, float>(args<float>(), fast_lists, stream);
+            enqueue_steps<float, float>(args<float>(), lists, 1, stream);
+            if (n_fast) enqueue_steps<float, float>(args<float>(), fast_lists, fast_k - 1, stream);
         }
     }
 

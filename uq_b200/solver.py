@@ -384,9 +384,9 @@ class Batch:
         """Kernels of one step taken phase by phase (profile, use_graph=False)."""
         return N.lib().lbm_batch_launches_per_step(self._h, 1 if residual else 0)
 
-    def graph_launches(self, residual=False):
-        """Kernels of one step replayed from a graph."""
-        return N.lib().lbm_batch_graph_launches(self._h, 1 if residual else 0)
+    def step_launches(self, n=1, residual=False):
+        """Kernels that step(n, residual) launches."""
+        return N.lib().lbm_batch_step_launches(self._h, int(n), 1 if residual else 0)
 
 
 class Server:
