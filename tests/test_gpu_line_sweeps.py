@@ -70,9 +70,10 @@ def test_fp64_tile_edges_match_oracle(cuda_device, flow, rk, fm):
 
 
 @pytest.mark.parametrize("prec", ["f32", "f64"])
-@pytest.mark.parametrize("rk,fm", [(1, 1), (0, 0), (2, 1), (3, 0)])
-def test_forms_of_a_step_agree_bit_for_bit(cuda_device, prec, rk, fm):
-    cases = [FLOWS[f](nx, ny, rkmethod=rk, fmethod=fm) for f in sorted(FLOWS) for nx, ny in SIZES[1:5]]
+@pytest.mark.parametrize("rks,fm", [((1,), 1), ((0,), 0), ((2,), 1), ((3,), 0), ((1, 0, 1, 2, 3), 1)])
+def test_forms_of_a_step_agree_bit_for_bit(cuda_device, prec, rks, fm):
+    pairs = [(f, size) for f in sorted(FLOWS) for size in SIZES[1:5]]
+    cases = [FLOWS[f](nx, ny, rkmethod=rks[k % len(rks)], fmethod=fm) for k, (f, (nx, ny)) in enumerate(pairs)]
     want, _ = _dists(cases, prec)
     for kw in (dict(tile=(16, 16)), dict(tile=(64, 4)), dict(use_graph=False)):
         got, _ = _dists(cases, prec, **kw)

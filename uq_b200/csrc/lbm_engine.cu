@@ -110,7 +110,7 @@ HostSample derive(const lbm_config &c, const lbm_init &in)
         throw LbmError(LBM_ERR_INVALID, "lbm_init tables missing");
     const int Nx = in.Nx, Ny = in.Ny;
     if (Nx < 3 || Ny < 3) throw LbmError(LBM_ERR_INVALID, "Nx and Ny must be at least 3");
-    // the kernels address a sample's 26 planes with 32-bit offsets
+    // the kernels address a sample's 13 planes of pairs with 32-bit offsets
     if ((long long)Ny * (((long long)Nx + 31) / 32 * 32) > (1ll << 26))
         throw LbmError(LBM_ERR_INVALID, "sample too large: Ny * roundup(Nx, 32) must be at most 2^26 nodes");
     s.nx = Nx;
@@ -217,7 +217,7 @@ void check_tile_shape(int x, int y)
 }
 
 // Sample parameters, rest state, node flags, wall list and spacing tables
-// of one sample; layout per sample: 26 planes of ny x pitch, pitch a
+// of one sample; layout per sample: 13 planes of (f, h) pairs, ny x pitch, pitch a
 // multiple of 32.
 void prepare_sample(const HostSample &h, int prec, PreparedSample &out)
 {
@@ -675,7 +675,7 @@ struct lbm_batch {
         CU(cudaGetDevice(&device));
         CU(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
 
-        // layout: per sample 26 planes of ny x pitch, packed one after another
+        // layout: per sample 13 planes of (f, h) pairs, ny x pitch, packed one after another
         std::vector<double> v_tdx, v_tdy, v_dx, v_dy, fref_host;
         std::vector<uint8_t> flags;
         long long state_off = 0, node_off = 0;

@@ -14,7 +14,6 @@
 // issues their copies, waits for them alone, and leaves the flux differences
 // in the box when it has read it.  The only block barrier comes before the
 // per-node stage or update.
-// What bounds it: see the measurements at k_flux.
 #pragma once
 
 #include "lbm_box.h"
@@ -524,14 +523,18 @@ struct NodeParts {
     }
 };
 
-// whether the per-node half loads the state before the block's barrier
+// Whether the per-node half loads the state before the block's barrier: the
+// loads then run while other warps sweep.  FP64 (3 % of a step, and flux_free
+// needs it) and RK1, which has registers for it; FP32 RK3 spills instead
+// (1.32 -> 1.36 ms per step of a 64-sample ensemble).
 template <class S>
 __host__ __device__ constexpr bool flux_early(int mode)
 {
     return sizeof(S) == 8 || mode == 3;
 }
 
-// FP64, ahead of the block's barrier: everything that needs no flux.  v is the
+// FP64, ahead of the block's barrier: everything that needs no flux (a 1024^2
+// step 0.471 -> 0.449 ms against forming it after the barrier).  v is the
 // state, and becomes the new value but for its flux term (RK3 stage 3: what
 // stage 3 relaxes from); m: the state's moment sums.  Whether the
 // equilibrium's mass check fails.
@@ -833,7 +836,12 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
     }
 }
 
-// blocks per SM that the registers leave room for
+// Blocks per SM.  FP32 RK3 stage 3 takes 128 registers and two blocks: at three
+// (160 bytes of spills) the kernel alone is 4 % faster, but a 64-sample
+// ensemble's step goes from 1.32 to 1.34 ms, the board being at its power
+// limit.  The other FP32 phases fit 80 registers and three blocks (the final
+// phase with the next step's stages 1.29 ms per step; at two 1.37; four
+// without them +1 %).  FP64 has no room for a third block's registers.
 template <class S, int MODE, bool SWEEP>
 struct FluxBlocks {
     static constexpr int value = !SWEEP || sizeof(S) == 8 ? 2 : MODE == 1 ? 2 : 3;
@@ -844,7 +852,20 @@ struct FluxBlocks {
 // PATH: FLUX_SWEEP or FLUX_GENERAL, the tiles of one kind per launch (a
 // block given the other kind returns at once).
 // TC: the default tile shape, compiled in; other shapes are read from the
-// arguments and give every node the same bits.
+// arguments and give every node the same bits (1024^2 Couette FP32, ms per
+// step: 0.31 compiled in, 0.48 to 0.58 for other shapes).
+// LAW: samples may have a viscosity law (macro_from_sums); only FP64 has
+// instances without (a 1001 x 101 plate 3 % faster, FP32 RK1 1 % slower).
+// NEXT: RK3's final phase goes on to the next step's stages (joins).
+//
+// What bounds it (64-sample ensemble, 3.5 M nodes; per-node sweeps with a
+// barrier per four directions before): FP32 stage 3 535 us, waits on
+// dependencies and loads at 16 warps per SM, issue slots 49 % used, FMA pipe
+// 47 %, DRAM 33 % at the 413 of 416 bytes a node it has to move; the final
+// phase with the next step's stages 380 us, issue slots 58 %, FMA pipe 56 %,
+// DRAM 45 %.  FP64 780 and 430 us, FP64 pipe 62 and 61 %, DRAM 50 and 59 %.
+// Steps of the same ensemble: FP32 1.98 -> 1.29 ms (5.1 M nodes), FP64 of 16
+// samples 1.99 -> 0.97 ms (2.2 M nodes).
 template <class S, int MODE, int PATH, bool TC, bool LAW, bool NEXT>
 __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP && TC>::value) k_flux(KArgs<S> a)
 {

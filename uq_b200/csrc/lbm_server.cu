@@ -12,7 +12,7 @@
 //
 // Device memory.  One arena of cap_nodes node slots; a solve holds
 // ny * pitch consecutive slots (pitch = nx rounded up to 32), which address
-// its 26 planes in each of the state, stage-2 and stage-3 buffers, its wall
+// its 13 planes of pairs in each of the state, stage-2 and stage-3 buffers, its wall
 // factors and its node flags exactly as a batch lays out one sample.  When a
 // solve retires its fields are written into its own stage-2 planes, which no
 // later step reads, and copied out from there.
@@ -224,7 +224,7 @@ struct lbm_server {
             if (frac > 0.9) frac = 0.9;
             arena_bytes = (size_t)(frac * (double)free_b);
         }
-        // per node slot: 26 planes in three buffers, the wall factor, the flags
+        // per node slot: 13 planes of pairs in three buffers, the wall factor, the flags
         const size_t per_node = 3 * NPL * es + es + 1;
         const long long cap = (long long)(arena_bytes / per_node) / 32 * 32;
         if (cap < 32 * 32) throw LbmError(LBM_ERR_NOMEM, "arena too small");
