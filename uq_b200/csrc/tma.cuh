@@ -81,9 +81,4 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map)
-{
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-
 }  // namespace uqlbm
