@@ -900,6 +900,9 @@ __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP &&
             pdl_wait();
             issue_warp<S>(t, maps, sm, bars, warp);
         }
+        // the warp's other lanes poll the barriers only once they are set up
+        // (the block barrier below is not on every path)
+        __syncwarp();
     } else if constexpr (SWEEP) {
         if (tid == 0) {
             for (int b = 0; b < a.slots; ++b) mbar_init(&bars[b], 1);
