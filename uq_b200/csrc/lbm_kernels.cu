@@ -314,19 +314,29 @@ __global__ void __launch_bounds__(IO_N) k_set_macro(const SampleParams *samples,
     });
 }
 
-// blocks for ns samples of up to `nodes` nodes each
-static dim3 io_grid(long long nodes, int ns)
+// calls f(grid, first sample) for ns samples of up to `nodes` nodes each, as
+// many in one launch as a grid holds along y
+template <class F>
+static cudaError_t io_launches(long long nodes, int s0, int ns, F f)
 {
     const long long tiles = (nodes + IO_N - 1) / IO_N + 1;
-    return dim3((unsigned)std::min<long long>(tiles, ns > 1 ? 256 : 2048), (unsigned)ns);
+    const unsigned x = (unsigned)std::min<long long>(tiles, ns > 1 ? 256 : 2048);
+    constexpr int MAX_Y = 65535;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < ns && e == cudaSuccess; k += MAX_Y) {
+        f(dim3(x, (unsigned)std::min(MAX_Y, ns - k)), s0 + k);
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 template <class S>
 cudaError_t launch_set_macro(const SampleParams *samples, int s0, int ns, S *state, S *buf2, S *buf3, const double *fields,
                              long long stride, const uint8_t *nflags, const double *fref, long long nodes, cudaStream_t st)
 {
-    k_set_macro<S><<<io_grid(nodes, ns), IO_N, 0, st>>>(samples, s0, ns > 1, state, buf2, buf3, fields, stride, nflags, fref);
-    return cudaGetLastError();
+    return io_launches(nodes, s0, ns, [&](dim3 grid, int s) {
+        k_set_macro<S><<<grid, IO_N, 0, st>>>(samples, s, ns > 1, state, buf2, buf3, fields, stride, nflags, fref);
+    });
 }
 template cudaError_t launch_set_macro<double>(const SampleParams *, int, int, double *, double *, double *, const double *,
                                               long long, const uint8_t *, const double *, long long, cudaStream_t);
@@ -372,16 +382,18 @@ template <class S>
 cudaError_t launch_macro_out(const SampleParams *samples, int s0, int ns, const S *state, double *out, long long stride,
                              long long nodes, cudaStream_t st)
 {
-    k_macro_out<S><<<io_grid(nodes, ns), IO_N, 0, st>>>(samples, s0, ns > 1, state, out, stride);
-    return cudaGetLastError();
+    return io_launches(nodes, s0, ns, [&](dim3 grid, int s) {
+        k_macro_out<S><<<grid, IO_N, 0, st>>>(samples, s, ns > 1, state, out, stride);
+    });
 }
 
 template <class S>
 cudaError_t launch_dist_io(const SampleParams *samples, int s, S *state, S *buf2, S *buf3, double *aos, int to_aos,
                            const uint8_t *nflags, const double *fref, long long nodes, cudaStream_t st)
 {
-    k_dist_io<S><<<io_grid(nodes, 1), IO_N, 0, st>>>(samples, s, state, buf2, buf3, aos, to_aos, nflags, fref);
-    return cudaGetLastError();
+    return io_launches(nodes, s, 1, [&](dim3 grid, int k) {
+        k_dist_io<S><<<grid, IO_N, 0, st>>>(samples, k, state, buf2, buf3, aos, to_aos, nflags, fref);
+    });
 }
 
 // Self-test of the bounded mbarrier wait the stencil kernels use: one block
