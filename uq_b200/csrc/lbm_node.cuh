@@ -121,8 +121,7 @@ struct Relax64 {
     {
         const double dt = xmul(w, sp.dt);  // m.q = 1/tau_f
         c = make_double2(xmul(dt, m.q), xmul(dt, xmul(sp.Pr, m.q)));
-        const double bx = xadd(1.0, c.x), by = xadd(1.0, c.y), r = rcp64(xmul(bx, by));
-        ic = make_double2(xmul(r, by), xmul(r, bx));
+        ic = make_double2(rcp64(xadd(1.0, c.x)), rcp64(xadd(1.0, c.y)));
         g = xmul(dt, xmul(xsub(sp.Pr, 1.0), m.q));
         cu = xmul(sp.c, m.ux);
         cv = xmul(sp.c, m.uy);
