@@ -5,6 +5,7 @@ the CPU-baseline leg of bench.py, never by the product package.
 """
 import ctypes as C
 import os
+import subprocess
 
 import numpy as np
 
@@ -106,6 +107,7 @@ class Oracle:
         for k, a in arrs.items():
             self._keep.append(a)
             setattr(ini, k, a.ctypes.data_as(_ip if a.dtype == np.int32 else _dp))
+        self.cfg, self.ini = cfg, ini
         self._h = L.orc_create(C.byref(cfg), C.byref(ini))
         if not self._h:
             raise ValueError("orc_create rejected the case")
@@ -165,3 +167,52 @@ def equilibrium(rho, ux, uy, T, R, Tc, K):
     eqf, eqh = np.empty(13), np.empty(13)
     lib().orc_equilibrium(rho, ux, uy, T, R, Tc, K, _d(eqf), _d(eqh))
     return eqf, eqh
+
+
+class Extended:
+    """One step of the same restatement in extended precision (x87, 64-bit
+    significands), from FP64 distributions: what an FP64 step's rounding
+    errors are measured against.  Built from the same source on first use."""
+
+    _lib = None
+
+    def __init__(self, case):
+        if Extended._lib is None:
+            subprocess.run(["make", "-s", "-C", HERE, "lib/liblbm_oracle_ext.so"], check=True)
+            Extended._lib = C.CDLL(os.path.join(HERE, "lib", "liblbm_oracle_ext.so"))
+            Extended._lib.orc_create.restype = C.c_void_p
+        base = Oracle(case)  # checked, its structures copied with every double widened
+        self.nx, self.ny = base.nx, base.ny
+        self._keep = []
+        cfg, ini = self._wide(base.cfg), self._wide(base.ini)
+        self._h = C.c_void_p(Extended._lib.orc_create(C.byref(cfg), C.byref(ini)))
+
+    def _wide(self, s):
+        kinds = {C.c_double: C.c_longdouble, _dp: C.POINTER(C.c_longdouble)}
+        wide = type("Wide", (C.Structure,), {"_fields_": [(k, kinds.get(t, t)) for k, t in s._fields_]})()
+        lengths = {"dx_array": self.nx, "dy_array": self.ny}
+        for k, t in s._fields_:
+            v = getattr(s, k)
+            if t is _dp and v:
+                v = np.ctypeslib.as_array(v, shape=(lengths.get(k) or s.numProps,)).astype(np.longdouble)
+                self._keep.append(v)
+                v = v.ctypes.data_as(kinds[_dp])
+            elif t is _dp:
+                continue
+            setattr(wide, k, v)
+        return wide
+
+    def step_from(self, f, h):
+        """f and h after one step from f, h, as extended-precision arrays."""
+        L, p = Extended._lib, lambda a: C.c_void_p(a.ctypes.data)
+        f, h = (np.ascontiguousarray(v, dtype=np.longdouble) for v in (f, h))
+        L.orc_set_dist(self._h, p(f), p(h))
+        L.orc_step(self._h, 1, 0, C.c_void_p(np.zeros(1, np.longdouble).ctypes.data))
+        fo, ho = np.empty_like(f), np.empty_like(h)
+        L.orc_get_dist(self._h, p(fo), p(ho))
+        return fo, ho
+
+    def __del__(self):
+        if getattr(self, "_h", None):
+            Extended._lib.orc_destroy(self._h)
+            self._h = None

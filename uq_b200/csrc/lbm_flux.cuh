@@ -657,12 +657,13 @@ __device__ __forceinline__ void node_phase(const KArgs<S> &a, const Tile &t, con
             // RK3 stage 3 and the part of the update that does not need the
             // stage-3 fluxes, from the moments of f - div F(f2)
             V *__restrict__ b3 = pair_base(a.buf3, sp) + o;
+            MomentSums md;
 #pragma unroll
             for (int i = 1; i < NQ; ++i) {
                 const V D = div(i);
-                m0.sub(i, D.x, D.y);
+                md.add(i, D.x, D.y);
             }
-            const Macro m3 = m0.template macro<LAW>(sp);
+            const Macro m3 = m0.less(md).template macro<LAW>(sp);
             EqArgs<C, DEV> q3(m3.rho, m3.ux, m3.uy, m3.T, sp);
             const Stage3Rest s(m3, sp);
             double sf3 = 0;
