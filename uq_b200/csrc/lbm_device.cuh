@@ -196,12 +196,13 @@ __device__ __forceinline__ float2 kc<float2>(double v) { return make_float2((flo
 template <>
 __device__ __forceinline__ double2 kc<double2>(double v) { return make_double2(v, v); }
 
-// FP64 reciprocal of a normal number: PTX's approximate reciprocal
-// (about 23 bits) and one third-order Newton (Chebyshev) step, y (1 + e + e^2)
-// with e = 1 - d y, whose error e^3 is below the FP64 rounding (measured: the
-// correctly rounded value or, rarely, its neighbour),
-// in a third of the operations of a division and without its branch for
-// special operands (a division per face was a fifth of the FP64 sweeps).
+// FP64 reciprocal of a normal number whose reciprocal is normal (zero and
+// infinity give NaN): PTX's approximate reciprocal, whose operand and result
+// have 20 fraction bits, and one cubic Newton (Chebyshev) step, y (1 + e + e^2)
+// with e = 1 - d y; |e| < 2^-18 leaves e^3 < 2^-54, so the result is the
+// correctly rounded one or its neighbour.  It takes a third of the operations
+// of a division and no branch for special operands (a division per face was a
+// fifth of the FP64 sweeps).
 __device__ __forceinline__ double rcp64(double d)
 {
     double y;
