@@ -471,7 +471,7 @@ struct lbm_batch {
     std::vector<int> tile_first, tile_count;
     long long total_state = 0, total_nodes = 0, lattice_nodes = 0;
     size_t max_nodes = 0;
-    bool any_rk3 = false, any_other = false, any_ghost = false;
+    bool any_rk3 = false, any_ghost = false;
 
     DevBuf<unsigned char> state, buf2, buf3, alpha;  // typed by precision
     DevBuf<uint8_t> nflags;
@@ -730,7 +730,7 @@ struct lbm_batch {
             node_off += p.plane;
             lattice_nodes += (long long)h.nx * h.ny;
             max_nodes = std::max(max_nodes, (size_t)h.nx * h.ny);
-            if (h.rk == 1) any_rk3 = true; else any_other = true;
+            if (h.rk == 1) any_rk3 = true;
             if (p.gx) any_ghost = true;
             sp.push_back(p);
         }

@@ -321,7 +321,7 @@ __device__ __forceinline__ void sweep_y(const Pair<S> *box, BoxPlace g, bool pos
 // (equal for the diagonals)
 template <class S, int FM>
 __device__ __forceinline__ bool sweep_warp(const Tile &t, const SampleParams &sp, const S *stage, Pair<S> *sm, S *save,
-                                           uint64_t *bars, uint32_t parity, int warp, int lane)
+                                           uint64_t *bars, int warp, int lane)
 {
     using V = Pair<S>;
     constexpr FluxSmem L = flux_smem<S>(TILE_CX, TILE_CY, true, true, 12);
@@ -336,7 +336,7 @@ __device__ __forceinline__ bool sweep_warp(const Tile &t, const SampleParams &sp
         const BoxPlace g = diag ? box_place<S>(BOX_XY, TILE_CX) : box_place<S>(BOX_X, TILE_CX);
         const bool pos = lat_ex(ix) > 0;
         const FaceArg<S> fa = face_arg<S>(t.c, t.eps1, lat_ex(ix));
-        ok = mbar_wait_bounded(&bars[ix - 1], parity, TMA_WAIT_POLLS);
+        ok = mbar_wait_bounded(&bars[ix - 1], 0, TMA_WAIT_POLLS);
         if (fix) {
             fix_box<S>(box, sp, stage, t, TILE_CX, TILE_CY, ix, lane, 32);
             __syncwarp();
@@ -354,7 +354,7 @@ __device__ __forceinline__ bool sweep_warp(const Tile &t, const SampleParams &sp
         const FaceArg<S> fa = face_arg<S>(t.c, t.eps1, lat_ey(iy));
         V out[8];
         if (!diag) {
-            ok = mbar_wait_bounded(&bars[iy - 1], parity, TMA_WAIT_POLLS) && ok;
+            ok = mbar_wait_bounded(&bars[iy - 1], 0, TMA_WAIT_POLLS) && ok;
             if (fix) {
                 fix_box<S>(box, sp, stage, t, TILE_CX, TILE_CY, iy, lane, 32);
                 __syncwarp();
@@ -483,13 +483,13 @@ __device__ __forceinline__ void face_parts(const Tile &t, const SampleParams &sp
 // the whole block of a default tile: each warp its directions
 template <class S>
 __device__ __forceinline__ bool sweep_tile(const Tile &t, const SampleParams &sp, const S *stage, Pair<S> *sm, S *save,
-                                           uint64_t *bars, uint32_t parity, int warp, int lane)
+                                           uint64_t *bars, int warp, int lane)
 {
     const int fm = tile_fm(t.kind);
     // FP64 has one form of the weights
-    if (sizeof(S) == 8 ? fm != 0 : fm == 1) return sweep_warp<S, 1>(t, sp, stage, sm, save, bars, parity, warp, lane);
-    if (fm == 2) return sweep_warp<S, sizeof(S) == 4 ? 2 : 1>(t, sp, stage, sm, save, bars, parity, warp, lane);
-    return sweep_warp<S, 0>(t, sp, stage, sm, save, bars, parity, warp, lane);
+    if (sizeof(S) == 8 ? fm != 0 : fm == 1) return sweep_warp<S, 1>(t, sp, stage, sm, save, bars, warp, lane);
+    if (fm == 2) return sweep_warp<S, sizeof(S) == 4 ? 2 : 1>(t, sp, stage, sm, save, bars, warp, lane);
+    return sweep_warp<S, 0>(t, sp, stage, sm, save, bars, warp, lane);
 }
 
 // a warp's lane 0 asks for the boxes of the warp's directions (maps: the stage
@@ -929,7 +929,7 @@ __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP &&
             if ((lane & 7) == 0 && t.y0 + warp < sp.ny)
                 for (int i = 0; i < NQ; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i * (int)sp.plane));
         }
-        ok = sweep_tile<S>(t, sp, stage, sm, save, bars, 0, warp, lane);
+        ok = sweep_tile<S>(t, sp, stage, sm, save, bars, warp, lane);
     } else if constexpr (SWEEP) {
         const int fm = tile_fm(t.kind), gx = (t.kind & TILE_GHOST) ? GHOST_X : 0;
         for (int i0 = 1, r = 0; i0 <= 12; i0 += a.slots, ++r) {

@@ -26,12 +26,6 @@ __device__ __forceinline__ float2 load_again(const float2 *p)
     asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
     return v;
 }
-__device__ __forceinline__ double2 load_again(const double2 *p)
-{
-    double2 v;
-    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-    return v;
-}
 
 // Ghost columns (SampleParams::gx): a node within gx of an x edge also
 // stores its stage-buffer values at its periodic image beyond the other
