@@ -503,7 +503,7 @@ struct EqArgs<C, false> {
     // Ends the sharing of subexpressions between the families before and
     // after it: kept for four families they are more registers than the few
     // products that form them again are worth (RK3 stage 3 spilled 850 bytes
-    // a thread, 240 so).
+    // a thread, 224 so).
     __device__ __forceinline__ void part() { asm volatile("" : "+d"(q.u), "+d"(q.v), "+d"(q.T), "+d"(q.K)); }
     __device__ __forceinline__ void fam(int f, C *fe, C *he) const
     {

@@ -854,7 +854,7 @@ struct FluxBlocks {
 // block given the other kind returns at once).
 // TC: the default tile shape, compiled in; other shapes are read from the
 // arguments and give every node the same bits (1024^2 Couette FP32, ms per
-// step: 0.31 compiled in, 0.48 to 0.58 for other shapes).
+// step: 0.28 compiled in, 0.48 to 0.57 for other shapes).
 // LAW: samples may have a viscosity law (macro_from_sums); only FP64 has
 // instances without (a 1001 x 101 plate 3 % faster, FP32 RK1 1 % slower).
 // NEXT: RK3's final phase goes on to the next step's stages (joins).
@@ -864,9 +864,9 @@ struct FluxBlocks {
 // dependencies and loads at 16 warps per SM, issue slots 49 % used, FMA pipe
 // 47 %, DRAM 33 % at the 413 of 416 bytes a node it has to move; the final
 // phase with the next step's stages 380 us, issue slots 58 %, FMA pipe 56 %,
-// DRAM 45 %.  FP64 780 and 430 us, FP64 pipe 62 and 61 %, DRAM 50 and 59 %.
+// DRAM 45 %.  FP64 789 and 433 us, FP64 pipe 62 and 61 %, DRAM 48 and 59 %.
 // Steps of the same ensemble: FP32 1.98 -> 1.29 ms (5.1 M nodes), FP64 of 16
-// samples 1.99 -> 0.97 ms (2.2 M nodes).
+// samples 1.99 -> 0.99 ms (2.2 M nodes).
 template <class S, int MODE, int PATH, bool TC, bool LAW, bool NEXT>
 __global__ void __launch_bounds__(256, FluxBlocks<S, MODE, PATH == FLUX_SWEEP && TC>::value) k_flux(KArgs<S> a)
 {
